@@ -601,24 +601,38 @@ HFG_API int hfg_op_project(const int res[3], const float spacing[3], float dt, c
           "rhs");
     // the CG kernels never store at non-fluid cells: both directions start zero
     check(cudaMemsetAsync(p1.p, 0, sizeof(float) * NC, s), "memset");
+    Scratch<int> sched(cgScheduleInts(cg), s);
+    check(launchCgSchedule(cg, cgc.p, sched.p, init.precond, false, s), "cg schedule");
     CgState host{};
+    auto readState = [&] {
+      check(cudaMemcpyAsync(&host, cs.p, sizeof(host), cudaMemcpyDeviceToHost, s), "read state");
+      check(cudaStreamSynchronize(s), "sync");
+    };
+    if (cgResidentEligible(cg, init.precond, false)) {
+      CoopLease lease(true);
+      Scratch<uint8_t> box(lease.held() ? cgResidentBytes(cg) : 0, s);
+      if (lease.held()) do {
+          check(launchCgResident(cg, sx, sy, sz, cgc.p, r.p, x.p, p0.p, p1.p, box.p, cs.p, init.precond, sched.p,
+                                 kResidentIters, s),
+                "resident cg");
+          readState();
+        } while (!host.done && host.resident == 1);
+    }
     float* pb[2] = {p0.p, p1.p};
     int it = 0;
-    for (;;) {
+    while (!host.done) {
       for (int k = 0; k < 16; ++k, ++it) {
         const int po = it & 1, pn = (it + 1) & 1;
         check(launchCgDirection(cg, sx, sy, sz, maps.rH, maps.pH[po], maps.codeH, cgc.p, r.p, pb[po], pb[pn], part.p,
-                                cs.p, init.precond, s),
+                                cs.p, init.precond, s, sched.p),
               "cg");
         check(launchCgUpdate(cg, sx, sy, sz, maps.pH[pn], maps.rI, maps.xI, maps.codeI, pb[pn], x.p, false, r.p, part.p,
-                             cs.p, init.precond, s),
+                             cs.p, init.precond, s, sched.p),
               "cg");
       }
-      check(cudaMemcpyAsync(&host, cs.p, sizeof(host), cudaMemcpyDeviceToHost, s), "read state");
-      check(cudaStreamSynchronize(s), "sync");
-      if (host.done) break;
+      readState();
     }
-    if (host.error) return fail(HFG_ERR_TIMEOUT, "pressure CG: a stage load did not complete in time");
+    if (host.error) return fail(HFG_ERR_TIMEOUT, "pressure CG: a wait did not complete in time");
     FaceField vv{{vx, vy, vz}};
     check(launchGradient(g, dt / (1.0f * spacing[0]), dt / (1.0f * spacing[1]), dt / (1.0f * spacing[2]), markers,
                          x.p, false, vv, sv, none, s),
@@ -659,6 +673,7 @@ int extrapolateGrids(int ngrids, const Dim3i* rc, float* const* vals, int layers
     User() { extrapUsers(+1); }
     ~User() { extrapUsers(-1); }
   } user;
+  CoopLease lease(false);
   check(launchExtrapLayers(r3, v3, off, sc, layers, s, nullptr), "extrapolation layers");
   unsigned int words[4] = {0, 0, 0, 0};
   check(cudaMemcpyAsync(words, extrapBarWords(sc), sizeof(words), cudaMemcpyDeviceToHost, s), "read");

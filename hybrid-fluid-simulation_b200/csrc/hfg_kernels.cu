@@ -7,7 +7,9 @@
 // The reference line each kernel follows is cited beside it.
 #include <algorithm>
 #include <atomic>
+#include <condition_variable>
 #include <cstdio>
+#include <mutex>
 
 #include "hfg_kernels.h"
 
@@ -611,6 +613,33 @@ namespace {
 std::atomic<int> g_extrapUsers{0};
 }
 void extrapUsers(int delta) { g_extrapUsers.fetch_add(delta); }
+
+namespace {
+std::mutex g_coopMu;
+std::condition_variable g_coopFree;
+int g_coopShared = 0;
+bool g_coopExclusive = false;
+}  // namespace
+
+CoopLease::CoopLease(bool exclusive) : exclusive_(exclusive), held_(true) {
+  std::unique_lock<std::mutex> lk(g_coopMu);
+  if (exclusive) {
+    held_ = !g_coopExclusive && g_coopShared == 0;
+    if (held_) g_coopExclusive = true;
+  } else {
+    g_coopFree.wait(lk, [] { return !g_coopExclusive; });
+    ++g_coopShared;
+  }
+}
+CoopLease::~CoopLease() {
+  if (!held_) return;
+  {
+    std::lock_guard<std::mutex> lk(g_coopMu);
+    if (exclusive_) g_coopExclusive = false;
+    else --g_coopShared;
+  }
+  g_coopFree.notify_all();
+}
 
 // Layers 1 .. nums-1 in one cooperative launch: about one block per 8192
 // faces of the grids, at most kExtrapPerSM per SM, and at most an equal

@@ -38,6 +38,7 @@ struct CgState {
   double tol;
   int error;        // nonzero: a kernel gave up (a stage load timed out); done is set too
   unsigned int ticket;  // last-block-done counter
+  int resident;         // launchCgResident: 1 it ran, 2 the system does not fit
 };
 
 // State of the CFL substep loop of one particle advection
@@ -178,6 +179,34 @@ constexpr int kCgTileX = 32, kCgTileY = 16;
 __host__ __device__ inline int schedItemsOffset(int cols) { return (2 * cols + 1 + 3) & ~3; }
 cudaError_t launchCgSchedule(const Dim3i& cg, const CgCode* code, int* sched, int precond, bool xDouble,
                              cudaStream_t s);
+// The resident CG (FP32 iterate, identity or Jacobi): up to maxIters
+// iterations of the solve in one cooperative launch, from and into the same
+// state, x, r and p as the kernel pair; zG is one more zeroed vector and
+// sched the solve's schedule (column extents).  CgState::resident tells
+// whether it ran.  The blocks wait on one another: launched under an
+// exclusive CoopLease only.
+constexpr int kResidentIters = 512;  // iterations the solvers ask of one launch
+bool cgResidentEligible(const Dim3i& cg, int precond, bool xDouble);
+// bytes of its mailboxes (16-byte aligned; cleared by every launch)
+size_t cgResidentBytes(const Dim3i& cg);
+cudaError_t launchCgResident(const Dim3i& cg, float sx, float sy, float sz, const CgCode* code, float* r, float* x,
+                             float* p, float* zG, void* mailboxes, CgState* st, int precond, const int* sched,
+                             int maxIters, cudaStream_t s);
+// Kernels whose blocks wait on one another must be resident together.  Those
+// that take a share of the GPU (launchExtrapLayers) hold a shared lease from
+// before the launch until the stream has been synchronised after it; one that
+// takes every SM holds the exclusive lease, which is only ever tried for.
+class CoopLease {
+ public:
+  explicit CoopLease(bool exclusive);  // shared: waits for an exclusive holder to finish
+  ~CoopLease();
+  bool held() const { return held_; }
+  CoopLease(const CoopLease&) = delete;
+  CoopLease& operator=(const CoopLease&) = delete;
+
+ private:
+  bool exclusive_, held_;
+};
 // Divergence residual of the projected velocity over the fluid cells:
 // *sumOut = sum b^2 (FP64), ticketAndMax[1] = bits of max |b|.  `scratch`
 // holds 2 * divergenceBlocks() doubles.

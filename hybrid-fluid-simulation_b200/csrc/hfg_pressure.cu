@@ -912,6 +912,625 @@ __global__ void __launch_bounds__(CTX* CTY, 4)
   }
 }
 
+// ---------------------------------------------------------------------------
+// The resident CG: whole solves in one cooperative launch, for systems whose
+// fluid fits the shared memory of the GPU.
+//
+// The kernel pair above streams r, p, x and the codes past every SM twice per
+// iteration and pays two launches, two ring fills and a block barrier per
+// plane for it; on small grids the launches alone are most of an iteration.
+// Here one block per SM keeps its share of the system for the whole solve:
+// p (with halo) and the codes in shared memory, and x, r and A p in registers
+// when the share is small (at most kResKL quads of cells to a thread), else x
+// and r stream from L2.  A thread works on four cells in x at a time, so the
+// addresses, the code test and the wide loads serve four.  An iteration is
+//   p = z + beta p on the block's cells and, from the neighbours' z, on its
+//     halo; A p; the grid reduction p.Ap -> alpha;
+//   x += alpha p, r -= alpha A p; z at the share's faces published to zG; the
+//     grid reductions r.r and r.z -> beta, and the stop test;
+// with the operations of kCgDirection and kCgUpdate on every cell, so the
+// iterates agree with theirs up to the order of the FP64 dot-product sums.
+// Every block sums the partials in the same fixed order and forms the same
+// scalars; the two grid reductions are the only waits (bounded at 2 s).
+//
+// Shares: the fluid runs of the tile columns (sched's extents) laid end to
+// end and cut into equal parts of n planes of 32 x 16 cells; a part covers
+// one or a few segments of columns, each with a halo plane at both ends.
+// A system whose parts do not fit leaves the state untouched (resident = 2)
+// and is solved by the kernel pair.
+// Measured (B200, Jacobi), us per iteration, pair -> resident: 33^3 dam break
+// 17.8 -> 6.9, 128^3 31.5 -> 10.4, 160^3 -> 15.6, 256^3 (4.0 M fluid cells)
+// 62 -> 34.  What bounds it now: the two reductions (about 2.5 us each) on the
+// small grids, issue slots (row sums, FP64 dot products) on the large ones.
+// 512 threads with up to 128 registers: 768 (80) and 1024 (64, spills) took 50
+// and 63 us at 256^3 where 512 took 45 (with one shared reduction array).
+constexpr int RTH = 512;                       // threads of a block
+constexpr int RQ = CTX / 4, RPT = RQ * CTR;    // a plane of a tile: 128 quads of 4 cells in x, one thread each
+constexpr int RG = RTH / RPT;                  // planes in hand at once
+static_assert(RQ == 8 && RTH % RPT == 0, "a warp holds four rows of eight quads");
+// A plane in shared memory: rows -1 .. 16 of 32 floats, then the columns left
+// and right of the tile (16 floats each).
+constexpr int RXL = (CTR + 2) * CTX, RXR = RXL + CTR, RPL = RXR + CTR;
+constexpr int kResPlanes = 96, kResSegs = 32;  // planes and segments of one block, at most
+constexpr int kResGrid = 256;                  // blocks, at most
+constexpr int kResMinPlanes = 2;
+constexpr int kResCols = 1024 / RTH;           // tile columns per thread of the share plan
+constexpr int kResKL = 4;                      // quads of a thread held in registers
+
+struct ResShared {
+  DiagTab tab;
+  int4 plane[kResPlanes];  // x0, y0, z, -
+  int2 at[kResPlanes];     // linear index of the tile origin; float offset of the plane | first or last of its segment
+  int4 seg[kResSegs];      // tile column, first plane, planes, first local plane
+  int segSlot[kResSegs];   // slot of the segment's lower halo plane
+  int hist[kResGrid];
+  double red[2][RTH / 32];
+  double tot[2][kResGrid / 32];
+  int scan[32];
+  int total, nSegs, maxSegs, ok;
+};
+
+// 16-byte accesses that other SMs see whole: a partial sum and its tag.
+struct Tagged {
+  double v;
+  unsigned long long tag;
+};
+__device__ __forceinline__ void putTagged(Tagged* p, double v, unsigned long long tag) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p),
+               "l"(__double_as_longlong(v)), "l"(tag)
+               : "memory");
+}
+__device__ __forceinline__ Tagged getTagged(const Tagged* p) {
+  Tagged r;
+  long long v;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(v), "=l"(r.tag)
+               : "l"(p)
+               : "memory");
+  r.v = __longlong_as_double(v);
+  return r;
+}
+
+// One grid reduction of a (and b) over blocks 0 .. m-1; every thread gets the
+// totals.  Every block has a mailbox with a slot for each block: a block puts
+// its partial sum, tagged with the epoch, into its slot of all m mailboxes and
+// polls its own.  So a reduction is one store and one load deep, and no line
+// is polled by more than one SM (with one shared array that all blocks polled,
+// an iteration took 13.5 us instead of 10.4 at 128^3).  The mailboxes of two
+// epochs alternate: a slot is written again only after every block has passed
+// the epoch between.  PUBLISH: global writes before the call are visible to
+// every block after it.  False once a wait ran out here or in another block.
+template <int NV, bool PUBLISH>
+__device__ __forceinline__ bool resReduce(double& a, double& b, ResShared& sh, Tagged* box, unsigned epoch, int m,
+                                          CgState* st) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  a = warpSumD(a);
+  if (NV > 1) b = warpSumD(b);
+  if (lane == 0) {
+    sh.red[0][w] = a;
+    if (NV > 1) sh.red[1][w] = b;
+  }
+  __syncthreads();
+  constexpr int U = kResGrid / 32;
+  static_assert(U <= RTH / 32 && RTH / 32 <= 32, "one warp per 32 blocks");
+  const unsigned long long tag = epoch + 1ull;
+  if (32 * w < m) {  // warp w serves blocks 32 w .. 32 w + 31
+    const int j = 32 * w + lane;
+    const double a0 = __shfl_sync(0xffffffffu, warpSumD(lane < RTH / 32 ? sh.red[0][lane] : 0.0), 0);
+    double b0 = 0.0;
+    if (NV > 1) b0 = __shfl_sync(0xffffffffu, warpSumD(lane < RTH / 32 ? sh.red[1][lane] : 0.0), 0);
+    // mailbox of block k: box[((epoch & 1) * m + k) * 2 m + ...]
+    Tagged* all = box + (size_t)(epoch & 1) * m * 2 * m;
+    if (j < m) {
+      if (PUBLISH) __threadfence();
+      Tagged* to = all + (size_t)j * 2 * m + blockIdx.x;
+      putTagged(to, a0, tag);
+      if (NV > 1) putTagged(to + m, b0, tag);
+    }
+    const Tagged* mine = all + (size_t)blockIdx.x * 2 * m;
+    Tagged v[NV];
+    unsigned long long deadline = 0;
+    for (int spin = 0;; ++spin) {
+      bool here = true;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        v[k] = Tagged{0.0, tag};
+        if (j < m) v[k] = getTagged(mine + k * m + j);
+      }
+#pragma unroll
+      for (int k = 0; k < NV; ++k) here = here && v[k].tag == tag;
+      if (__all_sync(0xffffffffu, here)) break;
+      if ((spin & 63) == 63) {
+        const unsigned long long now = globalNs();
+        if (deadline == 0) deadline = now + kWaitNs;
+        const bool give = now > deadline || ldAcquire((const unsigned*)&st->error) != 0u;
+        if (__any_sync(0xffffffffu, give)) {
+          if (lane == 0) {
+            cgFail(st, 2);
+            sh.ok = 0;
+          }
+          break;
+        }
+      }
+    }
+    if (PUBLISH) __threadfence();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const double sum = warpSumD(v[k].v);
+      if (lane == 0) sh.tot[k][w] = sum;
+    }
+  }
+  __syncthreads();
+  a = b = 0.0;
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (32 * u < m) {
+      a += sh.tot[0][u];
+      if (NV > 1) b += sh.tot[1][u];
+    }
+  return sh.ok != 0;
+}
+
+struct ResArgs {
+  Dim3i P;
+  float sx, sy, sz;
+  const CgCode* code;
+  float *r, *x, *p, *zG;
+  Tagged* box;
+  CgState* st;
+  int maxIters;  // iterations of this launch
+};
+
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+constexpr unsigned kAllInner = 0x7f7f7f7fu;  // four fluid cells, no neighbour solid or outside
+
+// Diagonals and reciprocals of four cells; a cell off the fluid has diagonal -1.
+__device__ __forceinline__ void diag4(const DiagTab& t, unsigned c4, float4& d, float4& inv) {
+  const float2 e = t.e[0x7f];
+  d = make_float4(e.x, e.x, e.x, e.x);
+  inv = make_float4(e.y, e.y, e.y, e.y);
+  if (c4 != kAllInner) {
+    const float2 e0 = t.e[c4 & 0xff], e1 = t.e[(c4 >> 8) & 0xff], e2 = t.e[(c4 >> 16) & 0xff], e3 = t.e[c4 >> 24];
+    d = make_float4(e0.x, e1.x, e2.x, e3.x);
+    inv = make_float4(e0.y, e1.y, e2.y, e3.y);
+  }
+}
+template <int PC>
+__device__ __forceinline__ float4 z4(float4 inv, float4 r) {
+  return make_float4(fastZ<PC>(inv.x, r.x), fastZ<PC>(inv.y, r.y), fastZ<PC>(inv.z, r.z), fastZ<PC>(inv.w, r.w));
+}
+__device__ __forceinline__ float4 fma4(float s, float4 a, float4 b) {
+  return make_float4(fmaf(s, a.x, b.x), fmaf(s, a.y, b.y), fmaf(s, a.z, b.z), fmaf(s, a.w, b.w));
+}
+// four rows of A (0 off the fluid)
+__device__ __forceinline__ float4 rows4(const ResArgs& A, float4 d, float4 c, float l, float r, float4 dn, float4 up,
+                                        float4 be, float4 ab) {
+  float4 q = make_float4(rowSum(d.x, A.sx, A.sy, A.sz, c.x, l, c.y, dn.x, up.x, be.x, ab.x),
+                         rowSum(d.y, A.sx, A.sy, A.sz, c.y, c.x, c.z, dn.y, up.y, be.y, ab.y),
+                         rowSum(d.z, A.sx, A.sy, A.sz, c.z, c.y, c.w, dn.z, up.z, be.z, ab.z),
+                         rowSum(d.w, A.sx, A.sy, A.sz, c.w, c.z, r, dn.w, up.w, be.w, ab.w));
+  if (d.x < 0.f) q.x = 0.f;
+  if (d.y < 0.f) q.y = 0.f;
+  if (d.z < 0.f) q.z = 0.f;
+  if (d.w < 0.f) q.w = 0.f;
+  return q;
+}
+__device__ __forceinline__ void dot4(double& s, float4 a, float4 b) {
+  s = fma((double)a.x, (double)b.x, s);
+  s = fma((double)a.y, (double)b.y, s);
+  s = fma((double)a.z, (double)b.z, s);
+  s = fma((double)a.w, (double)b.w, s);
+}
+
+// The solve of one block's share.  KL > 0: at most KL quads per thread, x, r
+// and A p in registers; KL = 0: any number, x and r in global memory and A p
+// formed twice.  Cells off the fluid hold zeros in every vector.
+template <int PC, int KL>
+__device__ void resSolve(const ResArgs& A, ResShared& sh, float* __restrict__ tile, const unsigned* __restrict__ codeS,
+                         int nb, int m) {
+  const int tid = threadIdx.x, grp = tid / RPT, cell = tid % RPT, row = cell / RQ, col = cell % RQ;
+  const Dim3i P = A.P;
+  CgState* st = A.st;
+  constexpr int KR = KL > 0 ? KL : 1, RU = 6;
+  float4 rR[KR], xR[KR], qR[KR];
+  const int nSegs = sh.nSegs;
+  // this thread's planes, its quad in a plane and the cells beside it
+  const int per = (nb + RG - 1) / RG, i0 = min(nb, grp * per), i1 = min(nb, i0 + per);
+  const int own = (row + 1) * CTX + 4 * col;
+  const int left = col == 0 ? RXL + row : own - 1, right = col == RQ - 1 ? RXR + row : own + 4;
+  const unsigned off = (unsigned)row * (unsigned)P.x + 4u * (unsigned)col;
+  const bool faceXY = row == 0 || row == CTR - 1 || col == 0 || col == RQ - 1;
+  float* __restrict__ gr = A.r;
+  float* __restrict__ gx = A.x;
+
+  // halo quads: rows -1 and 16 of every plane, then the halo planes of every segment
+  const int hq = 2 * RQ * nb, hAll = hq + 2 * RPT * nSegs;
+  auto haloQuad = [&](int h, int& t) -> int {
+    int gx0, gy, gz;
+    if (h < hq) {
+      const int i = h >> 4, hi = (h >> 3) & 1, c = h & 7;
+      const int4 pl = sh.plane[i];
+      gx0 = pl.x + 4 * c;
+      gy = hi ? pl.y + CTR : pl.y - 1;
+      gz = pl.z;
+      t = (sh.at[i].y & ~1) + (hi ? CTR + 1 : 0) * CTX + 4 * c;
+    } else {
+      const int k = h - hq, s = k >> 8, hi = (k >> 7) & 1, rw = (k >> 3) & 15, c = k & 7;
+      const int4 sg = sh.seg[s];
+      const int4 pl = sh.plane[sg.w];
+      gx0 = pl.x + 4 * c;
+      gy = pl.y + rw;
+      gz = hi ? sg.y + sg.z : sg.y - 1;
+      t = (sh.segSlot[s] + (hi ? sg.z + 1 : 0)) * RPL + (rw + 1) * CTX + 4 * c;
+    }
+    return gx0 < P.x && (unsigned)gy < (unsigned)P.y && (unsigned)gz < (unsigned)P.z ? (gz * P.y + gy) * P.x + gx0 : -1;
+  };
+  // halo columns: 16 cells left and 16 right of every plane
+  auto haloCol = [&](int h, int& t) -> int {
+    const int i = h >> 5, hi = (h >> 4) & 1, rw = h & 15;
+    const int4 pl = sh.plane[i];
+    const int gx1 = hi ? pl.x + CTX : pl.x - 1, gy = pl.y + rw;
+    t = (sh.at[i].y & ~1) + (hi ? RXR : RXL) + rw;
+    return (unsigned)gx1 < (unsigned)P.x && gy < P.y ? (pl.z * P.y + gy) * P.x + gx1 : -1;
+  };
+  auto publish = [&](int2 at, unsigned c, float4 z) {
+    if (faceXY || (at.y & 1)) __stcg(reinterpret_cast<float4*>(A.zG + c), z);
+  };
+
+  // the share as the last launch (or the RHS kernel) left it
+  for (int h = tid; h < hAll; h += RTH) {
+    int t;
+    const int g = haloQuad(h, t);
+    if (g >= 0) st4(tile + t, ld4(A.p + g));
+  }
+  for (int h = tid; h < 32 * nb; h += RTH) {
+    int t;
+    const int g = haloCol(h, t);
+    if (g >= 0) tile[t] = A.p[g];
+  }
+  for (int i = i0; i < i1; ++i) {
+    const unsigned c4 = codeS[i * RPT + cell];
+    if (!c4) continue;
+    const int2 at = sh.at[i];
+    const unsigned c = (unsigned)at.x + off;
+    float4 d, inv;
+    diag4(sh.tab, c4, d, inv);
+    st4(tile + (at.y & ~1) + own, ld4(A.p + c));
+    publish(at, c, z4<PC>(inv, ld4(gr + c)));
+  }
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (KL > 0) {
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+      rR[k] = xR[k] = qR[k] = zero;
+      if (i0 + k < i1 && codeS[(i0 + k) * RPT + cell]) {
+        const unsigned c = (unsigned)sh.at[i0 + k].x + off;
+        rR[k] = ld4(gr + c);
+        xR[k] = ld4(gx + c);
+      }
+    }
+  }
+  float beta = st->beta, alpha = st->alpha;
+  double rz = st->rz, rr = st->rr, pAp = st->pAp;
+  int iter = st->iter, done = 0;
+  const int maxIter = st->maxIter;
+  unsigned epoch = 0;
+  double a = 0.0, b = 0.0;
+  if (!resReduce<1, true>(a, b, sh, A.box, epoch++, m, st)) return;  // every share's z is out
+
+  for (int it = 0; it < A.maxIters; ++it) {
+    // p on the halo and on the share
+    for (int h0 = tid; h0 < hAll; h0 += 2 * RTH) {
+      float4 zv[2];
+      int t[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int h = h0 + u * RTH;
+        int g = -1;
+        if (h < hAll) g = haloQuad(h, t[u]);
+        if (g >= 0) zv[u] = __ldcg(reinterpret_cast<const float4*>(A.zG + g));
+        else t[u] = -1;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (t[u] >= 0) st4(tile + t[u], fma4(beta, ld4(tile + t[u]), zv[u]));
+    }
+    for (int h0 = tid; h0 < 32 * nb; h0 += 2 * RTH) {
+      float zv[2];
+      int t[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int h = h0 + u * RTH;
+        int g = -1;
+        if (h < 32 * nb) g = haloCol(h, t[u]);
+        if (g >= 0) zv[u] = __ldcg(A.zG + g);
+        else t[u] = -1;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (t[u] >= 0) tile[t[u]] = fmaf(beta, tile[t[u]], zv[u]);
+    }
+    if (KL > 0) {
+#pragma unroll
+      for (int k = 0; k < KR; ++k) {
+        if (i0 + k >= i1) continue;
+        const unsigned c4 = codeS[(i0 + k) * RPT + cell];
+        if (!c4) continue;
+        float4 d, inv;
+        diag4(sh.tab, c4, d, inv);
+        float* t = tile + (sh.at[i0 + k].y & ~1) + own;
+        st4(t, fma4(beta, ld4(t), z4<PC>(inv, rR[k])));
+      }
+    } else {
+      for (int ib = i0; ib < i1; ib += RU) {  // RU planes' loads in flight
+        unsigned c4[RU];
+        float4 rv[RU];
+#pragma unroll
+        for (int u = 0; u < RU; ++u) {
+          c4[u] = ib + u < i1 ? codeS[(ib + u) * RPT + cell] : 0u;
+          if (c4[u]) rv[u] = ld4(gr + (unsigned)sh.at[ib + u].x + off);
+        }
+#pragma unroll
+        for (int u = 0; u < RU; ++u) {
+          if (!c4[u]) continue;
+          float4 d, inv;
+          diag4(sh.tab, c4[u], d, inv);
+          float* t = tile + (sh.at[ib + u].y & ~1) + own;
+          st4(t, fma4(beta, ld4(t), z4<PC>(inv, rv[u])));
+        }
+      }
+    }
+    __syncthreads();
+    a = b = 0.0;
+    if (KL > 0) {
+#pragma unroll
+      for (int k = 0; k < KR; ++k) {
+        if (i0 + k >= i1) continue;
+        const unsigned c4 = codeS[(i0 + k) * RPT + cell];
+        if (!c4) continue;
+        float4 d, inv;
+        diag4(sh.tab, c4, d, inv);
+        const float* t = tile + (sh.at[i0 + k].y & ~1);
+        const float4 pc = ld4(t + own);
+        qR[k] = rows4(A, d, pc, t[left], t[right], ld4(t + own - CTX), ld4(t + own + CTX), ld4(t + own - RPL),
+                      ld4(t + own + RPL));
+        dot4(a, pc, qR[k]);
+      }
+    } else {
+      const float* tp = nullptr;
+      float4 be = zero, pc = zero;
+      for (int i = i0; i < i1; ++i) {
+        const float* t = tile + (sh.at[i].y & ~1);
+        if (t != tp) {  // the first plane of a segment
+          be = ld4(t + own - RPL);
+          pc = ld4(t + own);
+        }
+        const float4 ab = ld4(t + own + RPL);
+        const unsigned c4 = codeS[i * RPT + cell];
+        if (c4) {
+          float4 d, inv;
+          diag4(sh.tab, c4, d, inv);
+          dot4(a, pc, rows4(A, d, pc, t[left], t[right], ld4(t + own - CTX), ld4(t + own + CTX), be, ab));
+        }
+        be = pc;
+        pc = ab;
+        tp = t + RPL;
+      }
+    }
+    if (!resReduce<1, false>(a, b, sh, A.box, epoch++, m, st)) return;
+    pAp = a;
+    alpha = (float)(rz / pAp);
+    const bool skip = fabsf(alpha) < FLT_EPSILON;
+    a = b = 0.0;
+    if (KL > 0) {
+#pragma unroll
+      for (int k = 0; k < KR; ++k) {
+        if (i0 + k >= i1) continue;
+        const unsigned c4 = codeS[(i0 + k) * RPT + cell];
+        if (!c4) continue;
+        const int2 at = sh.at[i0 + k];
+        float4 d, inv;
+        diag4(sh.tab, c4, d, inv);
+        if (!skip) {
+          xR[k] = fma4(alpha, ld4(tile + (at.y & ~1) + own), xR[k]);
+          rR[k] = fma4(-alpha, qR[k], rR[k]);
+        }
+        const float4 zz = z4<PC>(inv, rR[k]);
+        publish(at, (unsigned)at.x + off, zz);
+        dot4(a, rR[k], rR[k]);
+        dot4(b, rR[k], zz);
+      }
+    } else {
+      const float* tp = nullptr;
+      float4 be = zero, pc = zero;
+      float4 rn = zero, xn = zero;  // r and x of the next plane, loaded one plane ahead
+      if (i0 < i1 && codeS[i0 * RPT + cell]) {
+        const unsigned c = (unsigned)sh.at[i0].x + off;
+        rn = ld4(gr + c);
+        xn = ld4(gx + c);
+      }
+      for (int i = i0; i < i1; ++i) {
+        const int2 at = sh.at[i];
+        const float* t = tile + (at.y & ~1);
+        float4 rv = rn, xv = xn;
+        if (i + 1 < i1 && codeS[(i + 1) * RPT + cell]) {
+          const unsigned c = (unsigned)sh.at[i + 1].x + off;
+          rn = ld4(gr + c);
+          xn = ld4(gx + c);
+        }
+        if (t != tp) {
+          be = ld4(t + own - RPL);
+          pc = ld4(t + own);
+        }
+        const float4 ab = ld4(t + own + RPL);
+        const unsigned c4 = codeS[i * RPT + cell];
+        if (c4) {
+          const unsigned c = (unsigned)at.x + off;
+          float4 d, inv;
+          diag4(sh.tab, c4, d, inv);
+          if (!skip) {
+            const float4 q = rows4(A, d, pc, t[left], t[right], ld4(t + own - CTX), ld4(t + own + CTX), be, ab);
+            st4(gx + c, fma4(alpha, pc, xv));
+            rv = fma4(-alpha, q, rv);
+            st4(gr + c, rv);
+          }
+          const float4 zz = z4<PC>(inv, rv);
+          publish(at, c, zz);
+          dot4(a, rv, rv);
+          dot4(b, rv, zz);
+        }
+        be = pc;
+        pc = ab;
+        tp = t + RPL;
+      }
+    }
+    if (!resReduce<2, true>(a, b, sh, A.box, epoch++, m, st)) return;
+    rr = a;
+    ++iter;
+    beta = (float)(b / rz);
+    rz = b;
+    done = cgStop(st, rr) || iter >= maxIter;
+    if (done) break;
+  }
+  // x for the caller; r and p for the next launch
+  if (KL > 0) {
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+      if (i0 + k < i1 && codeS[(i0 + k) * RPT + cell]) {
+        const unsigned c = (unsigned)sh.at[i0 + k].x + off;
+        st4(gx + c, xR[k]);
+        st4(gr + c, rR[k]);
+      }
+    }
+  }
+  if (!done)
+    for (int i = i0; i < i1; ++i)
+      if (codeS[i * RPT + cell]) {
+        const int2 at = sh.at[i];
+        st4(A.p + (unsigned)at.x + off, ld4(tile + (at.y & ~1) + own));
+      }
+  if (blockIdx.x == 0 && tid == 0) {
+    st->alpha = alpha;
+    st->beta = beta;
+    st->rz = rz;
+    st->rr = rr;
+    st->pAp = pAp;
+    st->iter = iter;
+    st->done = done;
+    st->resident = 1;
+  }
+}
+
+template <int PC>
+__global__ void __launch_bounds__(RTH, 1) kCgResident(ResArgs A, const int* __restrict__ sched, int cols, int dynBytes) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ __align__(16) ResShared sh;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  if (A.st->done) return;
+  buildDiagTab(sh.tab, A.sx, A.sy, A.sz);
+  // prefix sum of the columns' fluid planes, kResCols columns per thread
+  int lo[kResCols], len[kResCols], inc = 0;
+#pragma unroll
+  for (int j = 0; j < kResCols; ++j) {
+    const int c = kResCols * tid + j;
+    lo[j] = len[j] = 0;
+    if (c < cols) {
+      lo[j] = __ldg(sched + c);
+      const int hi = __ldg(sched + cols + c);
+      len[j] = hi >= lo[j] ? hi - lo[j] + 1 : 0;
+    }
+    inc += len[j];
+  }
+  const int mine = inc;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, d);
+    if (lane >= d) inc += v;
+  }
+  if (lane == 31) sh.scan[w] = inc;
+  for (int i = tid; i < kResGrid; i += RTH) sh.hist[i] = 0;
+  if (tid == 0) {
+    sh.nSegs = sh.maxSegs = 0;
+    sh.ok = 1;
+  }
+  __syncthreads();
+  if (w == 0) {
+    const int v = lane < RTH / 32 ? sh.scan[lane] : 0;
+    int vi = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, vi, d);
+      if (lane >= d) vi += u;
+    }
+    sh.scan[lane] = vi - v;
+    if (lane == 31) sh.total = vi;
+  }
+  __syncthreads();
+  const int S = sh.total, first = sh.scan[w] + inc - mine;
+  const int n = max(kResMinPlanes, (S + (int)gridDim.x - 1) / (int)gridDim.x);
+  const int m = (S + n - 1) / n;  // blocks with a share
+  // segments of every share: the fit is decided alike in every block
+  for (int j = 0, pre = first; j < kResCols; pre += len[j++])
+    if (len[j] > 0)
+      for (int b = pre / n; b <= (pre + len[j] - 1) / n; ++b) atomicMax(&sh.maxSegs, atomicAdd(&sh.hist[b], 1) + 1);
+  __syncthreads();
+  const int maxSegs = sh.maxSegs;
+  const long long need = (long long)(n + 2 * maxSegs) * RPL * sizeof(float) + (long long)n * (CTX * CTR);
+  if (n > kResPlanes || maxSegs > kResSegs || need > dynBytes) {
+    if (blockIdx.x == 0 && tid == 0) A.st->resident = 2;
+    return;
+  }
+  if ((int)blockIdx.x >= m) return;
+  // this block's segments, tile slots and planes
+  const int b0 = blockIdx.x * n, b1 = min(S, b0 + n), nb = b1 - b0;
+  for (int j = 0, pre = first; j < kResCols; pre += len[j++]) {
+    const int s0 = max(pre, b0), s1 = min(pre + len[j], b1);
+    if (len[j] > 0 && s0 < s1)
+      sh.seg[atomicAdd(&sh.nSegs, 1)] = make_int4(kResCols * tid + j, lo[j] + s0 - pre, s1 - s0, s0 - b0);
+  }
+  __syncthreads();
+  const int nSegs = sh.nSegs;
+  if (tid == 0) {
+    int slot = 0;
+    for (int s = 0; s < nSegs; ++s) {
+      sh.segSlot[s] = slot;
+      slot += sh.seg[s].z + 2;
+    }
+  }
+  __syncthreads();
+  const int tilesX = (A.P.x + CTX - 1) / CTX;
+  if (tid < nb) {
+    for (int s = 0; s < nSegs; ++s) {
+      const int4 sg = sh.seg[s];
+      const int k = tid - sg.w;
+      if (k < 0 || k >= sg.z) continue;
+      const int x0 = (sg.x % tilesX) * CTX, y0 = (sg.x / tilesX) * CTR, z = sg.y + k;
+      const int edge = k == 0 || k == sg.z - 1;
+      sh.plane[tid] = make_int4(x0, y0, z, 0);
+      sh.at[tid] = make_int2((z * A.P.y + y0) * A.P.x + x0, (sh.segSlot[s] + 1 + k) * RPL | edge);
+    }
+  }
+  float* tile = reinterpret_cast<float*>(dyn);
+  unsigned* codeS = reinterpret_cast<unsigned*>(tile + (n + 2 * maxSegs) * RPL);
+  for (int i = tid; i < (nb + 2 * nSegs) * RPL; i += RTH) tile[i] = 0.f;
+  __syncthreads();
+  for (int h = tid; h < nb * RPT; h += RTH) {
+    const int i = h / RPT, cell = h % RPT, row = cell / RQ, col = cell % RQ;
+    const int4 pl = sh.plane[i];
+    unsigned c4 = 0;
+    if (pl.x + 4 * col < A.P.x && pl.y + row < A.P.y)
+      c4 = __ldg(reinterpret_cast<const unsigned*>(A.code + (unsigned)sh.at[i].x + (unsigned)row * (unsigned)A.P.x +
+                                                   4u * (unsigned)col));
+    // cells off the fluid carry no bits, so four of them are code 0
+    const unsigned fl = c4 & 0x01010101u;
+    codeS[h] = c4 & (fl * 0xffu);
+  }
+  __syncthreads();
+  if ((n + RG - 1) / RG <= kResKL) resSolve<PC, kResKL>(A, sh, tile, codeS, nb, m);
+  else resSolve<PC, 0>(A, sh, tile, codeS, nb, m);
+}
+
 // Tensor map of a pitched 3-D array (x fastest) with the given box.
 cudaError_t encodeMap(CUtensorMap* m, const void* base, CUtensorMapDataType type, unsigned esize, const Dim3i& cg,
                       unsigned bx, unsigned by) {
@@ -967,6 +1586,43 @@ void cgWarmLaunchCache() {
   residentBlocks((const void*)kCgUpdate<0, double>);
   residentBlocks((const void*)kCgUpdate<1, double>);
   residentBlocks((const void*)kCgUpdate<2, double>);
+}
+
+bool cgResidentEligible(const Dim3i& cg, int precond, bool xDouble) {
+  return (precond == 0 || precond == 1) && !xDouble && cgColumns(cg) <= kResCols * RTH && cg.size() < (1ll << 30);
+}
+
+namespace {
+int residentGrid(const Dim3i& cg) {
+  const long long planes = (long long)cgColumns(cg) * cg.z;
+  return (int)std::max(1LL, std::min({(planes + kResMinPlanes - 1) / kResMinPlanes, (long long)numSMs(),
+                                      (long long)kResGrid}));
+}
+}  // namespace
+size_t cgResidentBytes(const Dim3i& cg) {
+  const size_t g = residentGrid(cg);
+  return 2 * g * 2 * g * sizeof(Tagged);
+}
+
+cudaError_t launchCgResident(const Dim3i& cg, float sx, float sy, float sz, const CgCode* code, float* r, float* x,
+                             float* p, float* zG, void* mailboxes, CgState* st, int precond, const int* sched,
+                             int maxIters, cudaStream_t s) {
+  const void* k = precond == 1 ? (const void*)kCgResident<1> : (const void*)kCgResident<0>;
+  int dev = 0, optin = 0;
+  cudaFuncAttributes fa{};
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k);
+  if (e != cudaSuccess) return e;
+  int dynBytes = (optin - (int)fa.sharedSizeBytes) & ~15;
+  if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dynBytes)) != cudaSuccess) return e;
+  int cols = cgColumns(cg);
+  const int grid = residentGrid(cg);
+  // the tags of an earlier launch must not look like this one's
+  if ((e = cudaMemsetAsync(mailboxes, 0, cgResidentBytes(cg), s)) != cudaSuccess) return e;
+  ResArgs A{cg, sx, sy, sz, code, r, x, p, zG, static_cast<Tagged*>(mailboxes), st, maxIters};
+  void* args[] = {&A, (void*)&sched, &cols, &dynBytes};
+  return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(RTH), args, (size_t)dynBytes, s);
 }
 
 int cgScheduleTarget(int precond, bool xDouble) {

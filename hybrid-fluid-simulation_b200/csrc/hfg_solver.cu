@@ -641,6 +641,33 @@ void GridSolver::runCg() {
             &cgGraph_[2], colZ_.p);
   } else {
     const int pc = opt_.precond == HFG_PRECOND_JACOBI ? 1 : 0;
+    if (!runCgResident(sx, sy, sz, pc)) runCgChunks(sx, sy, sz, pc);
+  }
+  if (cgHost_->error == 4) throw CudaError("pressure CG: a work item of the schedule is invalid", HFG_ERR_STATE);
+  if (cgHost_->error) throw CudaError("pressure CG: a wait did not complete in time", HFG_ERR_TIMEOUT);
+}
+
+// The solve in resident launches; false, with the system as it was, when
+// another kernel whose blocks wait on one another is in flight or the system
+// does not fit.
+bool GridSolver::runCgResident(float sx, float sy, float sz, int pc) {
+  if (!cgResidentEligible(cg_, pc, xDouble())) return false;
+  CoopLease lease(true);
+  if (!lease.held()) return false;
+  cgBox_.alloc(cgResidentBytes(cg_), stream_);
+  do {
+    launched(launchCgResident(cg_, sx, sy, sz, cgc_.p, cgr_.p, cgx_.p, cgp_[0].p, cgp_[1].p, cgBox_.p, cgState_.p,
+                              pc, colZ_.p, kResidentIters, stream_),
+             "resident cg");
+    readBack(cgHost_, cgState_.p, sizeof(CgState), stream_);
+    check(cudaStreamSynchronize(stream_), "cg sync");
+  } while (!cgHost_->done && cgHost_->resident == 1);
+  return cgHost_->done != 0;
+}
+
+// The solve in graph-replayed chunks of the streaming kernel pair.
+void GridSolver::runCgChunks(float sx, float sy, float sz, int pc) {
+  {
     // kCgChunk is even, so every chunk starts on the same p buffer
     if (!cgGraph_[pc])
       cgGraph_[pc] = capture([&] {
@@ -663,8 +690,6 @@ void GridSolver::runCg() {
     }
     cgChunks_ = (cgHost_->iter + kCgChunk - 1) / kCgChunk;
   }
-  if (cgHost_->error == 4) throw CudaError("pressure CG: a work item of the schedule is invalid", HFG_ERR_STATE);
-  if (cgHost_->error) throw CudaError("pressure CG: a stage load did not complete in time", HFG_ERR_TIMEOUT);
 }
 
 // PressureSolver.cpp:194-197 + GridFluidSolver.cpp:435-525
@@ -771,6 +796,7 @@ void GridSolver::extrapolate() {
     long long off[3] = {0, F_[0], F_[0] + F_[1]};
     ExtrapScratch sc{dist_.p, list_.p, hist_.p, offsets_.p, cursor_.p, mask_.p};
     launched(launchExtrapDistance(fr_, vals, off, nums, sc, stream_), "extrapolation distance", 17);
+    CoopLease lease(false);
     check(launchExtrapLayers(fr_, vals, off, sc, nums, stream_, &launches_), "extrapolation layers");
     readBack(extrapHost_, extrapBarWords(sc), sizeof(unsigned int) * 4, stream_);
     check(cudaStreamSynchronize(stream_), "extrapolation sync");

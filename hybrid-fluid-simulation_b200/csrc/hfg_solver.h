@@ -178,6 +178,8 @@ class GridSolver {
   void p2gCell(const float* vals, int span, int comp, float* out);
   void computePressure();
   void runCg();
+  bool runCgResident(float sx, float sy, float sz, int pc);
+  void runCgChunks(float sx, float sy, float sz, int pc);
   void cgIteration(int it, float sx, float sy, float sz, int pc);
   void autotuneCg(float sx, float sy, float sz, int pc);
   // Records what f() launches on the solver's stream as an executable graph.
@@ -225,6 +227,7 @@ class GridSolver {
   bool xDouble() const { return opt_.pressure_fp64 != 0; }
   void* xPtr() { return xDouble() ? (void*)cgx64_.p : (void*)cgx_.p; }
   DArray<double> partials_;
+  DArray<uint8_t> cgBox_;  // mailboxes of the resident CG
   DArray<int> colZ_;  // the CG schedule of the solve (launchCgSchedule)
   DArray<CgState> cgState_;
   CgState* cgHost_ = nullptr;  // pinned
