@@ -144,23 +144,6 @@ __device__ __forceinline__ void axisWeights(float t, int n, AxisW& a) {
   a.j = min(max(i, -1), n - 1);
 }
 
-// axisWeights with the coordinate clamped first to [-1, hi], hi the float
-// below n: the floor index is then in [-1, n - 1] with no integer clamp.  A
-// coordinate outside that range selects the same edge corners as the integer
-// clamp does, which hold equal values (the table's x differences and the y
-// and z corner pairs there are exact zeros), so every finite coordinate
-// samples the same value as with axisWeights; a NaN coordinate samples the
-// edge instead of returning NaN.
-__device__ __forceinline__ void clampedAxis(float t, float hi, int jmax, AxisW& a) {
-  const float c = fminf(fmaxf(t, -1.0f), hi);
-  const float f = floorf(c);
-  a.w1 = c - f;
-  const int i = (int)f;
-  a.i0 = max(i, 0);
-  a.i1 = min(i + 1, jmax);
-  a.j = i;
-}
-
 // Corner table of a face grid of nx x ny x nz values: (nx + 1) x (ny + 1) x
 // (nz + 2) float4, entry (L, jy, jx) = (f[z][y0][x0], f[z][y0][x1] -
 // f[z][y0][x0], f[z][y1][x0], f[z][y1][x1] - f[z][y1][x0]) with
@@ -180,12 +163,12 @@ struct FaceQuads {
   // Sampling constants of the grid, formed once on the host (makeFaceQuads)
   // so that a kernel reads them as launch parameters: the coordinate of a
   // point on axis k is p * inv + offF on the face grid of that axis and
-  // p * inv + offC (offF - 1/2) on the cell-centred one; hiF and hiC, the
-  // float below n + 1 and n for n cells, bound the coordinate on those two
-  // grids, and jF and jC (n and n - 1) are the largest floor index there;
-  // lx, ly and pl are the row length, the rows per layer and the layer size
-  // of component a's table.
-  float inv[3], offF[3], offC[3], hiF[3], hiC[3];
+  // p * inv + offC (offF - 1/2) on the cell-centred one; jF and jC (n and
+  // n - 1 for n cells) are the largest floor index there, and hi, the float
+  // below n + 1/2, bounds the face coordinate (QuadSampler); lx, ly and pl are
+  // the row length, the rows per layer and the layer size of component a's
+  // table.
+  float inv[3], offF[3], offC[3], hi[3];
   int jF[3], jC[3];
   unsigned lx[3], ly[3], pl[3];
 };
@@ -201,8 +184,7 @@ inline FaceQuads makeFaceQuads(const Geom& g, const float4* q0, const float4* q1
     q.offC[k] = q.offF[k] - 0.5f;
     q.jF[k] = n[k];
     q.jC[k] = n[k] - 1;
-    q.hiF[k] = std::nextafter((float)(n[k] + 1), 0.0f);
-    q.hiC[k] = std::nextafter((float)n[k], 0.0f);
+    q.hi[k] = std::nextafter((float)n[k] + 0.5f, 0.0f);
   }
   for (int a = 0; a < 3; ++a) {
     q.lx[a] = (unsigned)(n[0] + (a == 0) + 1);
@@ -235,12 +217,8 @@ struct FaceSampler {
     axisWeights(uz, g.r.z + 1, fc[2]);
   }
   // the same sampler from the constants of a corner-table set: one FMA per
-  // coordinate (the two forms round alike up to the last bit), and the
-  // coordinate clamped to [-1, n) before the floor (clampedAxis)
-  // The same with the integer index clamps of axisWeights (same corners and
-  // weights at every finite point): in the G2P kernel, which also forms the
-  // corner indices of the FLIP difference, this form is the faster one
-  // (1.03 against 1.19 ms per 256^3 step).
+  // coordinate (the two forms round alike up to the last bit), for the G2P
+  // kernel, which also forms the corner indices of the FLIP difference
   struct IndexClamp {};
   __device__ __forceinline__ FaceSampler(const FaceQuads& q, float px, float py, float pz, IndexClamp) {
     const float p[3] = {px, py, pz};
@@ -248,14 +226,6 @@ struct FaceSampler {
     for (int k = 0; k < 3; ++k) {
       axisWeights(fmaf(p[k], q.inv[k], q.offC[k]), q.jC[k] + 1, cc[k]);
       axisWeights(fmaf(p[k], q.inv[k], q.offF[k]), q.jF[k] + 1, fc[k]);
-    }
-  }
-  __device__ __forceinline__ FaceSampler(const FaceQuads& q, float px, float py, float pz) {
-    const float p[3] = {px, py, pz};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      clampedAxis(fmaf(p[k], q.inv[k], q.offC[k]), q.hiC[k], q.jC[k], cc[k]);
-      clampedAxis(fmaf(p[k], q.inv[k], q.offF[k]), q.hiF[k], q.jF[k], fc[k]);
     }
   }
   // weights and 8 linear indices of component `a` (corner order z, y, x);
@@ -298,25 +268,6 @@ struct FaceSampler {
     const float b0 = fmaf(wy, a01 - a00, a00), b1 = fmaf(wy, a11 - a10, a10);
     return fmaf(wz, b1 - b0, b0);
   }
-  // sampleQuads through the cache: the loads only when the entry differs
-  // from the cached one (or fresh)
-  __device__ __forceinline__ float sampleQuadsCached(const FaceQuads& T, int a, QuadCache& c, bool fresh) const {
-    const AxisW& X = a == 0 ? fc[0] : cc[0];
-    const AxisW& Y = a == 1 ? fc[1] : cc[1];
-    const AxisW& Z = a == 2 ? fc[2] : cc[2];
-    const int e = (Z.j * (int)T.ly[a] + Y.j) * (int)T.lx[a] + X.j;
-    if (fresh || e != c.e[a]) {
-      c.lo[a] = __ldg(T.c[a] + e);
-      c.hi[a] = __ldg(T.c[a] + e + T.pl[a]);
-      c.e[a] = e;
-    }
-    const float4 q0 = c.lo[a], q1 = c.hi[a];
-    const float wx = X.w1, wy = Y.w1, wz = Z.w1;
-    const float a00 = fmaf(wx, q0.y, q0.x), a01 = fmaf(wx, q0.w, q0.z);  // .y, .w: the x differences
-    const float a10 = fmaf(wx, q1.y, q1.x), a11 = fmaf(wx, q1.w, q1.z);
-    const float b0 = fmaf(wy, a01 - a00, a00), b1 = fmaf(wy, a11 - a10, a10);
-    return fmaf(wz, b1 - b0, b0);
-  }
   // sample of the difference field f - h at the same point
   __device__ __forceinline__ float sampleDiff(const Geom& g, int a, const float* __restrict__ f,
                                               const float* __restrict__ h) const {
@@ -336,16 +287,73 @@ __device__ __forceinline__ void sampleFaceFast(const ConstFaceField& v, const Ge
 #pragma unroll
   for (int a = 0; a < 3; ++a) out[a] = s.sample(g, a, v.c[a]);
 }
-__device__ __forceinline__ void sampleFaceQuads(const FaceQuads& v, float px, float py, float pz, float out[3]) {
-  FaceSampler s(v, px, py, pz);
+// The trilinear sample of the substeps, from the corner tables alone.  The
+// cell-centred coordinate of an axis is its face coordinate less 1/2, so one
+// floor per axis gives both base entries and weights: with w the face weight,
+// (j, w - 1/2) from the middle of a cell on, (j - 1, w + 1/2) before it (both
+// exact but for the last bit of the second).  The floor and its conversion run
+// on the quarter-rate pipe, and with one for each grid that pipe set the
+// substep's time: 48 of them per RK3 particle-substep, 24 now.  A 256^3 step
+// of 23 substeps of 31.4 M particles: 12.6 -> 11.5 ms; 160^3, 7.6 M: 132 ->
+// 124 us a launch.  (Resampling v0 instead of streaming it, 24 of the 48 bytes
+// a particle, cost 0.9 ms a step; no entry cache and 40 warps an SM cost 4.)
+// The coordinate is clamped first to [-1/2, n + 1/2): the bounds of both grids'
+// tables.  A coordinate outside selects the same edge corners as an integer
+// clamp would, which hold equal values (the x differences and the y and z
+// corner pairs there are exact zeros), so every finite point samples the same
+// value; a NaN point samples the edge instead of returning NaN.
+struct QuadSampler {
+  float wf[3], wc[3];
+  int jf[3], jc[3];
+  __device__ __forceinline__ QuadSampler(const FaceQuads& q, float px, float py, float pz) {
+    const float p[3] = {px, py, pz};
 #pragma unroll
-  for (int a = 0; a < 3; ++a) out[a] = s.sampleQuads(v, a);
+    for (int k = 0; k < 3; ++k) {
+      const float t = fminf(fmaxf(fmaf(p[k], q.inv[k], q.offF[k]), -0.5f), q.hi[k]);
+      const float f = floorf(t);
+      const float w = t - f;
+      const bool upper = w >= 0.5f;
+      jf[k] = (int)f;
+      jc[k] = upper ? jf[k] : jf[k] - 1;
+      wf[k] = w;
+      wc[k] = w + (upper ? -0.5f : 0.5f);
+    }
+  }
+  __device__ __forceinline__ int entry(const FaceQuads& T, int a) const {
+    const int X = a == 0 ? jf[0] : jc[0], Y = a == 1 ? jf[1] : jc[1], Z = a == 2 ? jf[2] : jc[2];
+    return (Z * (int)T.ly[a] + Y) * (int)T.lx[a] + X;
+  }
+  __device__ __forceinline__ float lerp(int a, const float4& q0, const float4& q1) const {
+    const float wx = a == 0 ? wf[0] : wc[0], wy = a == 1 ? wf[1] : wc[1], wz = a == 2 ? wf[2] : wc[2];
+    const float a00 = fmaf(wx, q0.y, q0.x), a01 = fmaf(wx, q0.w, q0.z);  // .y, .w: the x differences
+    const float a10 = fmaf(wx, q1.y, q1.x), a11 = fmaf(wx, q1.w, q1.z);
+    const float b0 = fmaf(wy, a01 - a00, a00), b1 = fmaf(wy, a11 - a10, a10);
+    return fmaf(wz, b1 - b0, b0);
+  }
+};
+__device__ __forceinline__ void sampleFaceQuads(const FaceQuads& v, float px, float py, float pz, float out[3]) {
+  const QuadSampler s(v, px, py, pz);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float4* q = v.c[a] + s.entry(v, a);
+    out[a] = s.lerp(a, __ldg(q), __ldg(q + v.pl[a]));
+  }
 }
+// through the cache: the loads only when the entry differs from the cached
+// one (or fresh)
 __device__ __forceinline__ void sampleFaceQuadsCached(const FaceQuads& v, float px, float py, float pz, float out[3],
                                                       QuadCache& c, bool fresh) {
-  FaceSampler s(v, px, py, pz);
+  const QuadSampler s(v, px, py, pz);
 #pragma unroll
-  for (int a = 0; a < 3; ++a) out[a] = s.sampleQuadsCached(v, a, c, fresh);
+  for (int a = 0; a < 3; ++a) {
+    const int e = s.entry(v, a);
+    if (fresh || e != c.e[a]) {
+      c.lo[a] = __ldg(v.c[a] + e);
+      c.hi[a] = __ldg(v.c[a] + e + v.pl[a]);
+      c.e[a] = e;
+    }
+    out[a] = s.lerp(a, c.lo[a], c.hi[a]);
+  }
 }
 
 // Cubic samplers (MPhysics/EulerMathTool.cu:134-240, FieldMathTool.cu:106-173).
