@@ -940,12 +940,9 @@ HFG_API int hfg_op_build_fluid_sdf(const int res[3], const float* domain, float*
     NEED(validRes(res) && domain && sdf && layers >= 1 && layers <= 100000, "invalid arguments");
     Dim3i r = toRes(res);
     cudaStream_t s = st(stream);
-    Scratch<unsigned int> fa(r.size(), s), fb(r.size(), s), cnt(2, s);
-    unsigned int* host = nullptr;
-    check(cudaMallocHost((void**)&host, sizeof(unsigned int)), "cudaMallocHost");
-    cudaError_t e = launchFluidSdf(r, domain, sdf, layers, fa.p, fb.p, cnt.p, host, s);
-    cudaFreeHost(host);
-    check(e, "fluid sdf");
+    Scratch<int> steps(r.size(), s);
+    Scratch<unsigned int> changed(kStepFlags, s);
+    check(launchFluidSdf(r, domain, sdf, layers, steps.p, changed.p, s), "fluid sdf");
     check(cudaStreamSynchronize(s), "sync");
     return HFG_OK;
   });
@@ -957,11 +954,11 @@ int fluidSideSdf(const int res[3], const float* density, const float* solid_sdf,
     NEED(validRes(res) && density && solid_sdf && out && distance >= 0 && distance <= 100000, "invalid arguments");
     Dim3i r = toRes(res);
     cudaStream_t s = st(stream);
-    Scratch<unsigned int> fa(r.size(), s), fb(r.size(), s), cnt(2, s);
-    unsigned int* host = nullptr;
-    check(cudaMallocHost((void**)&host, sizeof(unsigned int)), "cudaMallocHost");
-    cudaError_t e = launchFluidSideSdf(r, density, solid_sdf, outside, distance, out, fa.p, fb.p, cnt.p, host, s);
-    cudaFreeHost(host);
+    Scratch<int> steps(r.size(), s);
+    Scratch<unsigned int> changed(kStepFlags, s);
+    unsigned int* flags = (unsigned int*)pinnedGet(sizeof(unsigned int) * kStepFlags);
+    cudaError_t e = launchFluidSideSdf(r, density, solid_sdf, outside, distance, out, steps.p, changed.p, flags, s);
+    pinnedPut(flags);
     check(e, outside ? "fluid outside sdf" : "fluid inside sdf");
     check(cudaStreamSynchronize(s), "sync");
     return HFG_OK;

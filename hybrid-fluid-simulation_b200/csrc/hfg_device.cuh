@@ -292,8 +292,8 @@ __device__ __forceinline__ void sampleFaceFast(const ConstFaceField& v, const Ge
 // floor per axis gives both base entries and weights: with w the face weight,
 // (j, w - 1/2) from the middle of a cell on, (j - 1, w + 1/2) before it (both
 // exact but for the last bit of the second).  The floor and its conversion run
-// on the quarter-rate pipe, and with one for each grid that pipe set the
-// substep's time: 48 of them per RK3 particle-substep, 24 now.  A 256^3 step
+// on the quarter-rate pipe, which took 36 of them per RK3
+// particle-substep with one for each grid and takes 18 now.  A 256^3 step
 // of 23 substeps of 31.4 M particles: 12.6 -> 11.5 ms; 160^3, 7.6 M: 132 ->
 // 124 us a launch.  (Resampling v0 instead of streaming it, 24 of the 48 bytes
 // a particle, cost 0.9 ms a step; no entry cache and 40 warps an SM cost 4.)

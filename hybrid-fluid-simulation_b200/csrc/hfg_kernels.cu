@@ -687,51 +687,143 @@ cudaError_t launchCopyWords(const unsigned* src, unsigned* dst, int words, cudaS
 }
 
 // ===========================================================================
-// Fluid SDF of the fluid-domain field (buildFluidSDF, EulerSolverTool.cu:324-406,
-// :760-785; GridFluidSolver.cpp:571-591).  Layer 0 marks the cells on both
-// sides of the fluid surface (0.5 - 0.2 inside, 1.5 - 0.2 outside, +/-UNKNOWN
-// elsewhere); layer d then takes every still-UNKNOWN neighbour of a layer d-1
-// cell of the same side.  The reference sweeps the whole grid 1000 times;
-// here each layer visits only the previous layer's cells (frontier lists).
+// Distance fields in cells (buildFluidSDF and the hybrid coupler's inside /
+// outside fields below): the number of 6-neighbour steps from a set of seed
+// cells, some cells closed to the walk.  The reference grows the field one
+// step per sweep of the whole grid, up to 1000 of them.  Here the distances
+// relax along whole lines: one pass each along x, y and z (a forward and a
+// backward min(d, d_before + 1) sweep, stopping at closed cells) is a round.
+// With no closed cell one round gives every distance (the separable L1
+// transform); otherwise a cell at distance d is right after as many rounds as
+// its shortest walk has straight pieces at most, and a round that changes
+// nothing ends it: the passes are exact at their fixed point.  A few rounds
+// replace a launch and a host read per distance step: density, the three
+// distance fields and a field mix on 96^3 7.0 -> 0.36 ms.
 // ===========================================================================
 namespace {
 constexpr double kSurf = 0.2;  // FluidSurfaceDensity (Common.h:244)
 __device__ __forceinline__ float outsideValue(int d) { return (float)((double)d + (1.5 - kSurf)); }
 __device__ __forceinline__ float insideValue(int d) { return d == 0 ? (float)(0.5 - kSurf) : (float)(-((double)d - (0.5 - kSurf))); }
+constexpr int kStepsFar = 0x7fffff00, kStepsClosed = -1;
+constexpr int kStepRounds = kStepFlags;  // rounds between host reads, at most
 }  // namespace
 
-__global__ void kFluidSdfInit(Dim3i r, const float* __restrict__ dom, float* __restrict__ sdf,
-                              unsigned int* __restrict__ front, unsigned int* __restrict__ count) {
+// A pass of round `round` does nothing once an earlier round changed nothing.
+__device__ __forceinline__ bool stepsDone(const unsigned* changed, int round) {
+  return round > 0 && *(volatile const unsigned*)(changed + round - 1) == 0u;
+}
+
+// Along x: one warp per row, 32 cells at a time; a sweep is a warp prefix-min
+// of d - lane between closed cells, plus the carry of the chunk before.
+__global__ void kStepsRows(Dim3i r, int* __restrict__ d, unsigned* changed, int round) {
+  if (stepsDone(changed, round)) return;
+  const int lane = threadIdx.x & 31, rows = r.y * r.z, nw = (int)(gridDim.x * blockDim.x) >> 5;
+  bool any = false;
+  for (int row = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += nw) {
+    int* q = d + (size_t)row * r.x;
+#pragma unroll
+    for (int back = 0; back < 2; ++back) {
+      int carry = kStepsFar;
+      for (int s0 = 0; s0 < r.x; s0 += 32) {
+        const int j = s0 + lane, i = back ? r.x - 1 - j : j;
+        const int v = j < r.x ? q[i] : kStepsClosed;
+        const unsigned closed = __ballot_sync(0xffffffffu, v < 0);
+        // the last closed lane up to this one (-1: none)
+        const int wall = 31 - __clz((int)(closed & (0xffffffffu >> (31 - lane))));
+        int a = v < 0 ? kStepsFar : v - lane;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, a, o);
+          if (lane - o > wall) a = min(a, t);
+        }
+        int f = v < 0 ? kStepsFar : min(a + lane, kStepsFar);
+        if (wall < 0) f = min(f, carry + lane + 1);
+        if (v >= 0 && f < v) {
+          q[i] = f;
+          any = true;
+        }
+        carry = __shfl_sync(0xffffffffu, f, 31);
+      }
+      __syncwarp();
+    }
+  }
+  if (any) *(volatile unsigned*)(changed + round) = 1u;
+}
+
+// Along y (axis 1) or z: one thread per line, coalesced across x, the loads of
+// B cells in flight together.
+__global__ void kStepsCols(Dim3i r, int axis, int* __restrict__ d, unsigned* changed, int round) {
+  if (stepsDone(changed, round)) return;
+  const size_t nx = (size_t)r.x, plane = nx * r.y, stride = axis == 1 ? nx : plane;
+  const int len = axis == 1 ? r.y : r.z;
+  const size_t lines = axis == 1 ? nx * r.z : plane;
+  bool any = false;
+  for (size_t l = blockIdx.x * (size_t)blockDim.x + threadIdx.x; l < lines; l += (size_t)gridDim.x * blockDim.x) {
+    int* col = d + (axis == 1 ? (l / nx) * plane + l % nx : l);
+    constexpr int B = 16;
+#pragma unroll
+    for (int back = 0; back < 2; ++back) {
+      int prev = kStepsFar;
+      for (int s0 = 0; s0 < len; s0 += B) {
+        int v[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+          const int j = s0 + k;
+          v[k] = j < len ? col[(size_t)(back ? len - 1 - j : j) * stride] : kStepsClosed;
+        }
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+          const int j = s0 + k;
+          if (v[k] >= 0 && prev + 1 < v[k]) {
+            v[k] = prev + 1;
+            col[(size_t)(back ? len - 1 - j : j) * stride] = v[k];
+            any = true;
+          }
+          prev = v[k] < 0 ? kStepsFar : v[k];
+        }
+      }
+    }
+  }
+  if (any) *(volatile unsigned*)(changed + round) = 1u;
+}
+
+namespace {
+// The passes of rounds [from, to).
+cudaError_t launchStepRounds(const Dim3i& r, int* d, unsigned* changed, int from, int to, cudaStream_t s) {
+  for (int k = from; k < to; ++k) {
+    kStepsRows<<<gridFor((long long)r.y * r.z * 32), kThreads, 0, s>>>(r, d, changed, k);
+    kStepsCols<<<gridFor((long long)r.x * r.z, 64), 64, 0, s>>>(r, 1, d, changed, k);
+    kStepsCols<<<gridFor((long long)r.x * r.y, 64), 64, 0, s>>>(r, 2, d, changed, k);
+  }
+  return cudaGetLastError();
+}
+}  // namespace
+
+// Fluid SDF of the fluid-domain field (EulerSolverTool.cu:324-406, :760-785;
+// GridFluidSolver.cpp:571-591).  The cells on both sides of the fluid surface
+// are the seeds (0.5 - 0.2 inside, 1.5 - 0.2 outside); the field grows from
+// them on its own side only, which needs no closed cells: the surface cell
+// nearest to a cell lies on the cell's own side, and so does every shortest
+// walk to it.
+__global__ void kFluidSdfSeed(Dim3i r, const float* __restrict__ dom, int* __restrict__ d) {
   HFG_FOR(c, r.size()) {
     int x, y, z;
     cellCoord(c, r, x, y, z);
-    bool in = dom[c] < 0.f;
+    const bool in = dom[c] < 0.f;
     bool mixed = false;
     const int dx[6] = {-1, 1, 0, 0, 0, 0}, dy[6] = {0, 0, -1, 1, 0, 0}, dz[6] = {0, 0, 0, 0, -1, 1};
 #pragma unroll
     for (int k = 0; k < 6; ++k) mixed |= ((dom[linc(x + dx[k], y + dy[k], z + dz[k], r)] < 0.f) != in);
-    float v = in ? (mixed ? insideValue(0) : -kUnknown) : (mixed ? outsideValue(0) : kUnknown);
-    sdf[c] = v;
-    if (mixed) front[atomicAdd(count, 1u)] = (unsigned int)c;
+    d[c] = mixed ? 0 : kStepsFar;
   }
 }
-
-__global__ void kFluidSdfLayer(Dim3i r, float* __restrict__ sdf, const unsigned int* __restrict__ front,
-                               unsigned int n, unsigned int* __restrict__ next, unsigned int* __restrict__ count, int d) {
-  HFG_FOR(i, (long long)n) {
-    long long c = front[i];
-    int x, y, z;
-    cellCoord(c, r, x, y, z);
-    bool inside = sdf[c] < 1.0f;  // inner values are <= 0.3, outer >= 1.3
-    float sentinel = inside ? -kUnknown : kUnknown;
-    float v = inside ? insideValue(d) : outsideValue(d);
-    const int dx[6] = {-1, 1, 0, 0, 0, 0}, dy[6] = {0, 0, -1, 1, 0, 0}, dz[6] = {0, 0, 0, 0, -1, 1};
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      long long nb = linc(x + dx[k], y + dy[k], z + dz[k], r);
-      int old = atomicCAS((int*)(sdf + nb), __float_as_int(sentinel), __float_as_int(v));
-      if (old == __float_as_int(sentinel)) next[atomicAdd(count, 1u)] = (unsigned int)nb;
-    }
+__global__ void kFluidSdfValue(long long n, const float* __restrict__ dom, const int* __restrict__ d, int layers,
+                               float* __restrict__ sdf) {
+  HFG_FOR(c, n) {
+    const bool in = dom[c] < 0.f;
+    const int k = d[c];
+    const bool reached = k == 0 || k < layers;
+    sdf[c] = in ? (reached ? insideValue(k) : -kUnknown) : (reached ? outsideValue(k) : kUnknown);
   }
 }
 
@@ -837,30 +929,13 @@ cudaError_t launchMixParticleVel(const float* pic, const float* flip, const floa
   return cudaGetLastError();
 }
 
-cudaError_t launchFluidSdf(const Dim3i& r, const float* dom, float* sdf, int layers, unsigned int* frontA,
-                           unsigned int* frontB, unsigned int* counts, unsigned int* hostCount, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(unsigned int) * 2, s);
+cudaError_t launchFluidSdf(const Dim3i& r, const float* dom, float* sdf, int layers, int* steps, unsigned int* changed,
+                           cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(changed, 0, sizeof(unsigned int) * kStepFlags, s);
   if (e != cudaSuccess) return e;
-  kFluidSdfInit<<<gridFor(r.size()), kThreads, 0, s>>>(r, dom, sdf, frontA, counts);
-  unsigned int* cur = frontA;
-  unsigned int* nxt = frontB;
-  int slot = 0;
-  for (int d = 1; d < layers; ++d) {
-    e = cudaMemcpyAsync(hostCount, counts + slot, sizeof(unsigned int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return e;
-    unsigned int n = *hostCount;
-    if (n == 0) break;
-    e = cudaMemsetAsync(counts + (slot ^ 1), 0, sizeof(unsigned int), s);
-    if (e != cudaSuccess) return e;
-    kFluidSdfLayer<<<gridFor(n), kThreads, 0, s>>>(r, sdf, cur, n, nxt, counts + (slot ^ 1), d);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    unsigned int* t = cur;
-    cur = nxt;
-    nxt = t;
-    slot ^= 1;
-  }
+  kFluidSdfSeed<<<gridFor(r.size()), kThreads, 0, s>>>(r, dom, steps);
+  if ((e = launchStepRounds(r, steps, changed, 0, 1, s)) != cudaSuccess) return e;
+  kFluidSdfValue<<<gridFor(r.size()), kThreads, 0, s>>>(r.size(), dom, steps, layers, sdf);
   return cudaGetLastError();
 }
 
@@ -871,51 +946,35 @@ cudaError_t launchFluidSdf(const Dim3i& r, const float* dom, float* sdf, int lay
 // surface cells (density 0.2) the seed value s (0.2 - 0.5 inside, 0.5 - 0.2
 // outside), cells of density 0 (inside) or 1 (outside) 0 and the rest
 // UNKNOWN; sweep d then gives every UNKNOWN 6-neighbour of a cell holding
-// d - 1 + s the value d + s, and negative values end as 0.  The reference
-// sweeps the whole grid `distance` times; here each sweep visits the
-// previous shell only (frontier lists, as launchFluidSdf).
+// d - 1 + s the value d + s, and negative values end as 0.  So the surface
+// cells are the seeds and the cells that sweep 0 sets to 0 are closed.
 // ===========================================================================
 namespace {
 __device__ __forceinline__ bool realEq(float a, float b) { return fabsf(__fsub_rn(a, b)) < FLT_MIN; }  // isRealEQ
 }  // namespace
 
-__global__ void kSideSdfInit(Dim3i r, const float* __restrict__ density, const float* __restrict__ solid,
-                             float seed, float zero, float* __restrict__ out, unsigned int* __restrict__ front,
-                             unsigned int* __restrict__ count) {
-  HFG_FOR(c, r.size()) {
+__global__ void kSideSdfSeed(long long n, const float* __restrict__ density, const float* __restrict__ solid,
+                             float zero, int* __restrict__ d) {
+  HFG_FOR(c, n) {
     const float rho = density[c];
+    int v = kStepsFar;
+    if (solid[c] < 0.f) v = kStepsClosed;
+    else if (realEq(rho, (float)kSurf)) v = 0;
+    else if (realEq(rho, zero)) v = kStepsClosed;
+    d[c] = v;
+  }
+}
+// the value of every cell, buildFluidSDFPostProcess (HybridSimulatorBuildSDF.cu:122-137) included
+__global__ void kSideSdfValue(long long n, const int* __restrict__ d, double seed, int sweeps,
+                              float* __restrict__ out) {
+  HFG_FOR(c, n) {
+    const int k = d[c];
     float v = kUnknown;
-    bool surface = false;
-    if (solid[c] < 0.f) {
-      v = 0.f;
-    } else if (realEq(rho, (float)kSurf)) {
-      v = seed;
-      surface = true;
-    } else if (realEq(rho, zero)) {
-      v = 0.f;
-    }
+    if (k < 0) v = 0.f;
+    else if (k < sweeps) v = fmaxf((float)((double)k + seed), 0.f);
     out[c] = v;
-    if (surface) front[atomicAdd(count, 1u)] = (unsigned int)c;
   }
 }
-
-__global__ void kSideSdfLayer(Dim3i r, float* __restrict__ out, const unsigned int* __restrict__ front, unsigned int n,
-                              unsigned int* __restrict__ next, unsigned int* __restrict__ count, float v) {
-  HFG_FOR(i, (long long)n) {
-    const long long c = front[i];
-    int x, y, z;
-    cellCoord(c, r, x, y, z);
-    const int dx[6] = {-1, 1, 0, 0, 0, 0}, dy[6] = {0, 0, -1, 1, 0, 0}, dz[6] = {0, 0, 0, 0, -1, 1};
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      const long long nb = linc(x + dx[k], y + dy[k], z + dz[k], r);
-      const int old = atomicCAS((int*)(out + nb), __float_as_int(kUnknown), __float_as_int(v));
-      if (old == __float_as_int(kUnknown)) next[atomicAdd(count, 1u)] = (unsigned int)nb;
-    }
-  }
-}
-
-// buildFluidSDFPostProcess (HybridSimulatorBuildSDF.cu:122-137)
 __global__ void kNegativeToZero(long long n, float* __restrict__ out) {
   HFG_FOR(i, n) {
     if (out[i] < 0.f) out[i] = 0.f;
@@ -923,38 +982,32 @@ __global__ void kNegativeToZero(long long n, float* __restrict__ out) {
 }
 
 cudaError_t launchFluidSideSdf(const Dim3i& r, const float* density, const float* solid, bool outside, int distance,
-                               float* out, unsigned int* frontA, unsigned int* frontB, unsigned int* counts,
-                               unsigned int* hostCount, cudaStream_t s) {
-  // the reference's UInt + double expressions, rounded to Real once
-  const double seed = outside ? 0.5 - kSurf : kSurf - 0.5;
-  if (distance > 0) {
-    cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(unsigned int) * 2, s);
-    if (e != cudaSuccess) return e;
-    kSideSdfInit<<<gridFor(r.size()), kThreads, 0, s>>>(r, density, solid, (float)seed, outside ? 1.f : 0.f, out,
-                                                         frontA, counts);
-    unsigned int* cur = frontA;
-    unsigned int* nxt = frontB;
-    int slot = 0;
-    for (int d = 1; d < distance; ++d) {
-      // sweep d looks for (d + s) - 1; where that is not the value sweep
-      // d - 1 wrote, the reference's shell stops growing
-      if ((float)((double)d + seed - 1) != (float)((double)(d - 1) + seed)) break;
-      e = cudaMemcpyAsync(hostCount, counts + slot, sizeof(unsigned int), cudaMemcpyDeviceToHost, s);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-      if (e != cudaSuccess) return e;
-      const unsigned int n = *hostCount;
-      if (n == 0) break;
-      e = cudaMemsetAsync(counts + (slot ^ 1), 0, sizeof(unsigned int), s);
-      if (e != cudaSuccess) return e;
-      kSideSdfLayer<<<gridFor(n), kThreads, 0, s>>>(r, out, cur, n, nxt, counts + (slot ^ 1),
-                                                   (float)((double)d + seed));
-      e = cudaGetLastError();
-      if (e != cudaSuccess) return e;
-      std::swap(cur, nxt);
-      slot ^= 1;
-    }
+                               float* out, int* steps, unsigned int* changed, unsigned int* hostFlags,
+                               cudaStream_t s) {
+  if (distance <= 0) {
+    kNegativeToZero<<<gridFor(r.size()), kThreads, 0, s>>>(r.size(), out);
+    return cudaGetLastError();
   }
-  kNegativeToZero<<<gridFor(r.size()), kThreads, 0, s>>>(r.size(), out);
+  // the reference's UInt + double expressions, rounded to Real once; sweep d
+  // looks for (d + s) - 1, and where that is not the value sweep d - 1 wrote,
+  // the reference's shell stops growing
+  const double seed = outside ? 0.5 - kSurf : kSurf - 0.5;
+  int sweeps = 1;
+  while (sweeps < distance && (float)((double)sweeps + seed - 1) == (float)((double)(sweeps - 1) + seed)) ++sweeps;
+  kSideSdfSeed<<<gridFor(r.size()), kThreads, 0, s>>>(r.size(), density, solid, outside ? 1.f : 0.f, steps);
+  // three rounds see most scenes through (walks around a convex solid have
+  // two or three pieces); then as many again as have been done
+  bool settled = false;
+  for (int rounds = 3; !settled; rounds = std::min(2 * rounds, kStepRounds)) {
+    cudaError_t e = cudaMemsetAsync(changed, 0, sizeof(unsigned int) * kStepFlags, s);
+    if (e == cudaSuccess) e = launchStepRounds(r, steps, changed, 0, rounds, s);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(hostFlags, changed, sizeof(unsigned int) * rounds, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return e;
+    settled = hostFlags[rounds - 1] == 0u;
+  }
+  kSideSdfValue<<<gridFor(r.size()), kThreads, 0, s>>>(r.size(), steps, seed, sweeps, out);
   return cudaGetLastError();
 }
 

@@ -264,18 +264,20 @@ inline unsigned int* extrapBarWords(const ExtrapScratch& sc) { return sc.hist + 
 // operator call); the launch sizes its grid to a share of the GPU per user.
 void extrapUsers(int delta);
 
-// ---- fluid SDF (buildFluidSDF); frontier buffers hold N cells each; counts 2;
-// hostCount pinned.  Blocks (one host read per layer).
+// ---- distance fields --------------------------------------------------------
+// steps: one int per cell; changed: kStepFlags words.
+constexpr int kStepFlags = 48;
+// fluid SDF of a fluid-domain field (buildFluidSDF); asynchronous
+cudaError_t launchFluidSdf(const Dim3i& r, const float* domain, float* sdf, int layers, int* steps,
+                           unsigned int* changed, cudaStream_t s);
 // The hybrid coupler's inside / outside distance fields of a fluid density
-// (frontier lists of r.size() entries each, two counters, one pinned host
-// word; the stream is synchronised once per sweep) and its mixed outside field.
+// (hostFlags: kStepFlags pinned words; the stream is synchronised once per
+// few relaxation rounds) and its mixed outside field.
 cudaError_t launchFluidSideSdf(const Dim3i& r, const float* density, const float* solid, bool outside, int distance,
-                               float* out, unsigned int* frontA, unsigned int* frontB, unsigned int* counts,
-                               unsigned int* hostCount, cudaStream_t s);
+                               float* out, int* steps, unsigned int* changed, unsigned int* hostFlags,
+                               cudaStream_t s);
 cudaError_t launchMixedOutsideSdf(const Dim3i& r, const float* gridDensity, const float* mixedDensity,
                                   const float* gridOutside, float* out, cudaStream_t s);
-cudaError_t launchFluidSdf(const Dim3i& r, const float* dom, float* sdf, int layers, unsigned int* frontA,
-                           unsigned int* frontB, unsigned int* counts, unsigned int* hostCount, cudaStream_t s);
 // mixFieldWithDensity of a cell grid (face = 0, a[0], b[0]) or of the three
 // face grids of r (face = 1); b is updated in place
 cudaError_t launchMixFieldWithDensity(const Dim3i& r, int face, const float* const a[3], float* const b[3],

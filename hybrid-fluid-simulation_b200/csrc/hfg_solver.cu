@@ -996,15 +996,12 @@ void GridSolver::getSolidVel(float* x, float* y, float* z) {
 // GridFluidSolver.cpp:571-591 generateCurFluidSDF on the current domain field
 void GridSolver::getFluidSDF(float* out) {
   DArray<float> sdf;
-  DArray<unsigned int> fa, fb, cnt;
+  DArray<int> steps;
+  DArray<unsigned int> changed;
   sdf.alloc(N_, stream_);
-  fa.alloc(N_, stream_);
-  fb.alloc(N_, stream_);
-  cnt.alloc(2, stream_);
-  unsigned int* host = (unsigned int*)pinnedGet(sizeof(unsigned int));
-  cudaError_t e = launchFluidSdf(g_.r, dom_[cur()].p, sdf.p, opt_.extrapolation_layers, fa.p, fb.p, cnt.p, host, stream_);
-  pinnedPut(host);
-  check(e, "fluid sdf");
+  steps.alloc(N_, stream_);
+  changed.alloc(kStepFlags, stream_);
+  check(launchFluidSdf(g_.r, dom_[cur()].p, sdf.p, opt_.extrapolation_layers, steps.p, changed.p, stream_), "fluid sdf");
   check(cudaMemcpyAsync(out, sdf.p, N_ * 4, cudaMemcpyDeviceToHost, stream_), "download");
   synchronize();
 }
