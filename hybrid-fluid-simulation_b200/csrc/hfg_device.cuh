@@ -281,12 +281,67 @@ struct FaceSampler {
   }
 };
 
-__device__ __forceinline__ void sampleFaceFast(const ConstFaceField& v, const Geom& g, float px, float py, float pz,
-                                               float out[3]) {
-  FaceSampler s(g, px, py, pz);
-#pragma unroll
-  for (int a = 0; a < 3; ++a) out[a] = s.sample(g, a, v.c[a]);
+// Trilinear sampling of the face grids and of cell fields at one point without
+// corner tables (semi-Lagrangian advection, LINEAR G2P).  The cell-centred
+// coordinate of an axis is its face coordinate less 1/2, so one floor per axis
+// serves both grids (as in QuadSampler), and a sample is seven lerps.  The
+// coordinate is clamped to [-1/2, n + 1/2) first, where the corners are the
+// edge ones already; a coordinate that is not finite makes every weight, and
+// so every sample, NaN.
+struct LerpGrid {
+  float inv[3], o[3], hi[3];
+  int n[3];
+};
+inline LerpGrid makeLerpGrid(const Geom& g) {
+  LerpGrid q;
+  const float h[3] = {g.hx, g.hy, g.hz}, o[3] = {g.ox, g.oy, g.oz};
+  const int n[3] = {g.r.x, g.r.y, g.r.z};
+  for (int k = 0; k < 3; ++k) {
+    q.inv[k] = 1.0f / h[k];
+    q.o[k] = o[k];
+    q.hi[k] = std::nextafter((float)n[k] + 0.5f, 0.0f);
+    q.n[k] = n[k];
+  }
+  return q;
 }
+struct LerpSampler {
+  float wf[3], wc[3];
+  int f0[3], f1[3], c0[3], c1[3];
+  __device__ __forceinline__ LerpSampler(const LerpGrid& q, float px, float py, float pz) {
+    const float p[3] = {px, py, pz};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float u = (p[k] - q.o[k]) * q.inv[k];
+      const float t = fminf(fmaxf(u, -0.5f), q.hi[k]);
+      const float f = floorf(t);
+      const float w = (t - f) + (u - u);
+      const bool upper = !(w < 0.5f);
+      const int j = (int)f, jc = upper ? j : j - 1;
+      wf[k] = w;
+      wc[k] = w + (upper ? -0.5f : 0.5f);
+      f0[k] = max(j, 0);
+      f1[k] = min(j + 1, q.n[k]);
+      c0[k] = max(jc, 0);
+      c1[k] = min(jc + 1, q.n[k] - 1);
+    }
+  }
+  // component a of a face field (0-2) or a cell field (3)
+  __device__ __forceinline__ float sample(const LerpGrid& q, int a, const float* __restrict__ f) const {
+    const unsigned nx = (unsigned)(q.n[0] + (a == 0)), ny = (unsigned)(q.n[1] + (a == 1));
+    const unsigned x0 = a == 0 ? f0[0] : c0[0], x1 = a == 0 ? f1[0] : c1[0], y0 = a == 1 ? f0[1] : c0[1],
+                   y1 = a == 1 ? f1[1] : c1[1];
+    const unsigned r0 = (unsigned)(a == 2 ? f0[2] : c0[2]) * ny, r1 = (unsigned)(a == 2 ? f1[2] : c1[2]) * ny;
+    const float wx = a == 0 ? wf[0] : wc[0], wy = a == 1 ? wf[1] : wc[1], wz = a == 2 ? wf[2] : wc[2];
+    const unsigned b00 = (r0 + y0) * nx, b01 = (r0 + y1) * nx, b10 = (r1 + y0) * nx, b11 = (r1 + y1) * nx;
+    const float v0 = __ldg(f + (b00 + x0)), v1 = __ldg(f + (b00 + x1)), v2 = __ldg(f + (b01 + x0)),
+                v3 = __ldg(f + (b01 + x1)), v4 = __ldg(f + (b10 + x0)), v5 = __ldg(f + (b10 + x1)),
+                v6 = __ldg(f + (b11 + x0)), v7 = __ldg(f + (b11 + x1));
+    const float a00 = fmaf(wx, v1 - v0, v0), a01 = fmaf(wx, v3 - v2, v2);
+    const float a10 = fmaf(wx, v5 - v4, v4), a11 = fmaf(wx, v7 - v6, v6);
+    const float d0 = fmaf(wy, a01 - a00, a00), d1 = fmaf(wy, a11 - a10, a10);
+    return fmaf(wz, d1 - d0, d0);
+  }
+};
 // The trilinear sample of the substeps, from the corner tables alone.  The
 // cell-centred coordinate of an axis is its face coordinate less 1/2, so one
 // floor per axis gives both base entries and weights: with w the face weight,
