@@ -357,70 +357,79 @@ bool marchLevel0(const Dim3i& r) {
 }
 
 // Residual of level f restricted to level c: bc = mean over the children of
-// (b - A z).
+// (b - A z).  Two lanes to a coarse cell, one for each x of its children: the
+// loads run along fine rows, and a lane's chain is four children long instead
+// of eight (64^3 level 0: 7.9 -> 6.2 us).
+constexpr int RX = 32, RYZ = 4;  // a block: 16 coarse cells in x, 4 in y, 2 in z
+dim3 restrictGrid(const Dim3i& rc) { return dim3((rc.x + 15) / 16, (rc.y + RYZ - 1) / RYZ, (rc.z + 1) / 2); }
 template <class TB, class TZ, class TBC>
 __global__ void kResidualRestrict(Lvl Lf, Dim3i rc, const TB* __restrict__ b, const TZ* __restrict__ zf,
                                   const Code* __restrict__ code, TBC* __restrict__ bc, const CgState* st) {
   waitPrevGrid();
   if (st->done) return;
   allowNextGrid();
-  int X, Y, Z;
-  unsigned C;
-  if (!cellOf(rc, X, Y, Z, C)) return;
+  const int x = blockIdx.x * RX + threadIdx.x;  // fine
+  const int Y = blockIdx.y * RYZ + threadIdx.y, Z = blockIdx.z * 2 + threadIdx.z;
+  const unsigned nx = (unsigned)Lf.r.x, pl = nx * (unsigned)Lf.r.y;
   float s = 0.f;
-  for (int kk = 0; kk < 2; ++kk)
-    for (int j = 0; j < 2; ++j)
-      for (int i = 0; i < 2; ++i) {
-        int x = 2 * X + i, y = 2 * Y + j, z = 2 * Z + kk;
-        if (x >= Lf.r.x || y >= Lf.r.y || z >= Lf.r.z) continue;
-        unsigned c = ((unsigned)z * Lf.r.y + y) * Lf.r.x + x;
-        Code k = code[c];
-        if (!(k & 1)) continue;
-        const unsigned pl = (unsigned)Lf.r.x * Lf.r.y;
-        float az = applyA(Lf, k, ld(zf, c), [&](int d) {
-          int dx, dy, dz;
-          nbrOf(d, dx, dy, dz);
-          return ld(zf, c + dx + dy * Lf.r.x + dz * pl);
-        });
-        s += ld(b, c) - az;
-      }
-  bc[C] = cvt<TBC>(0.125f * s);
+  if (x < Lf.r.x && Y < rc.y && Z < rc.z) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int y = 2 * Y + (q & 1), z = 2 * Z + (q >> 1);
+      if (y >= Lf.r.y || z >= Lf.r.z) continue;
+      const unsigned c = ((unsigned)z * Lf.r.y + y) * nx + x;
+      const Code k = code[c];
+      if (!(k & 1)) continue;
+      const float az = applyA(Lf, k, ld(zf, c), [&](int d) {
+        int dx, dy, dz;
+        nbrOf(d, dx, dy, dz);
+        return ld(zf, c + dx + dy * nx + dz * pl);
+      });
+      s += ld(b, c) - az;
+    }
+  }
+  s += __shfl_down_sync(0xffffffffu, s, 1);
+  const int X = x >> 1;
+  if (!(threadIdx.x & 1) && X < rc.x && Y < rc.y && Z < rc.z)
+    bc[((unsigned)Z * rc.y + Y) * rc.x + X] = cvt<TBC>(0.125f * s);
 }
 
-// Coarsest level: Jacobi sweeps in one block's shared memory.
+// Coarsest level: Jacobi sweeps in one block's shared memory.  One cell to a
+// thread: its code, right-hand side, diagonal and value stay in registers, the
+// sweep reads the neighbours only, and the warps that hold cells meet on a
+// barrier of their own.  A chain of kCoarseSweeps sweeps, so latency is all of
+// it: 17.8 -> 13.1 us for 512 cells.
+static_assert(kCoarseMax <= 1024 && kCoarseSweeps % 2 == 0, "a cell to a thread; the result's buffer");
 template <class TB, class TZ>
-__global__ void kCoarseSolve(Lvl L, const TB* __restrict__ b, TZ* __restrict__ z, const Code* __restrict__ code,
-                             const CgState* st) {
+__global__ void __launch_bounds__(kCoarseMax)
+    kCoarseSolve(Lvl L, const TB* __restrict__ b, TZ* __restrict__ z, const Code* __restrict__ code,
+                 const CgState* st) {
   waitPrevGrid();
   if (st->done) return;
   allowNextGrid();
-  __shared__ float za[kCoarseMax], zb[kCoarseMax];
-  unsigned n = (unsigned)L.r.size();
-  for (unsigned c = threadIdx.x; c < n; c += blockDim.x) za[c] = 0.f;
-  __syncthreads();
-  float* cur = za;
-  float* nxt = zb;
+  __shared__ float zs[2][kCoarseMax];
+  const int n = (int)L.r.size(), c = threadIdx.x, active = (n + 31) & ~31;
+  if (c >= active) return;
+  const bool mine = c < n;
+  const Code k = mine ? code[c] : (Code)0;
+  const float bv = mine ? ld(b, (unsigned)c) : 0.f, diag = diagOfC(k, L.sx, L.sy, L.sz);
+  const int pl = L.r.x * L.r.y;
+  float v = 0.f;
+  zs[0][c] = 0.f;
   for (int it = 0; it < kCoarseSweeps; ++it) {
-    for (unsigned c = threadIdx.x; c < n; c += blockDim.x) {
-      Code k = code[c];
-      float v = 0.f;
-      if (k & 1) {
-        const unsigned pl = (unsigned)L.r.x * L.r.y;
-        float az = applyA(L, k, cur[c], [&](int d) {
-          int dx, dy, dz;
-          nbrOf(d, dx, dy, dz);
-          return cur[c + dx + dy * L.r.x + dz * pl];
-        });
-        v = cur[c] + kOmega * (ld(b, c) - az) / diagOfC(k, L.sx, L.sy, L.sz);
-      }
-      nxt[c] = v;
+    asm volatile("bar.sync 1, %0;" ::"r"(active) : "memory");
+    const float* cur = zs[it & 1];
+    if (k & 1) {
+      const float az = applyA(L, k, v, [&](int d) {
+        int dx, dy, dz;
+        nbrOf(d, dx, dy, dz);
+        return cur[c + dx + dy * L.r.x + dz * pl];
+      });
+      v = v + kOmega * (bv - az) / diag;
     }
-    __syncthreads();
-    float* t = cur;
-    cur = nxt;
-    nxt = t;
+    zs[(it + 1) & 1][c] = v;
   }
-  for (unsigned c = threadIdx.x; c < n; c += blockDim.x) z[c] = cvt<TZ>(cur[c]);
+  if (mine) z[c] = cvt<TZ>(v);
 }
 }  // namespace
 
@@ -445,6 +454,7 @@ struct Multigrid {
   DArray<double> partials;
   CUtensorMap zH[2], pH[2];          // halo tensor maps of z0a / z0b and p[0] / p[1]
   long long chunkLaunches = 0;       // kernels in one captured chunk of CG iterations
+  int chunks = 0;                    // chunks the last solve needed
   const Code* code0 = nullptr;
   float s0[3] = {0, 0, 0};
   ~Multigrid() {
@@ -548,7 +558,7 @@ const float* vcycleT(Multigrid* m, const float* r0, CgState* st, cudaStream_t s,
     lv[l] = Lvl{m->res[l], m->s0[0] * f, m->s0[1] * f, m->s0[2] * f};
   }
   auto codeOf = [&](int l) -> const Code* { return l == 0 ? m->code0 : m->code[l - 1]->p; };
-  const dim3 blk(BX, BY, BZ);
+  const dim3 blk(BX, BY, BZ), rblk(RX, RYZ, 2);
   const int nu = m->smooth;
   // every kernel of the V-cycle is a programmatic dependent launch: the launch
   // of the next one overlaps the tail of this one
@@ -586,7 +596,7 @@ const float* vcycleT(Multigrid* m, const float* r0, CgState* st, cudaStream_t s,
         march(kJacobiZ<float, false, false, BF, BF>, lv[0], lv[0].r, r0, (const BF*)hz[cb], hz[cb ^ 1],
               (const float*)nullptr, codeOf(0), (double*)nullptr, st);
       curBuf[0] = cb;
-      run(kResidualRestrict<float, BF, TS>, gridOf(lv[1].r), blk, lv[0], lv[1].r, r0, (const BF*)hz[cb], codeOf(0),
+      run(kResidualRestrict<float, BF, TS>, restrictGrid(lv[1].r), rblk, lv[0], lv[1].r, r0, (const BF*)hz[cb], codeOf(0),
           bL[1], (const CgState*)st);
     } else if (l == 0) {
       if (marching)
@@ -603,7 +613,7 @@ const float* vcycleT(Multigrid* m, const float* r0, CgState* st, cudaStream_t s,
                 z0[cb ^ 1], (const float*)nullptr, codeOf(0), (double*)nullptr, st);
       }
       curBuf[0] = cb;
-      run(kResidualRestrict<float, float, TS>, gridOf(lv[1].r), blk, lv[0], lv[1].r, r0, (const float*)z0[cb],
+      run(kResidualRestrict<float, float, TS>, restrictGrid(lv[1].r), rblk, lv[0], lv[1].r, r0, (const float*)z0[cb],
           codeOf(0), bL[1], (const CgState*)st);
     } else {
       TS* zl[2] = {zaL[l], zbL[l]};
@@ -613,7 +623,7 @@ const float* vcycleT(Multigrid* m, const float* r0, CgState* st, cudaStream_t s,
         sweep(kJacobi<TS, TS, TS, false, false>, lv[l].r, false, lv[l], lv[l].r, (const TS*)bL[l], (const TS*)zl[cb],
               zl[cb ^ 1], (const TS*)nullptr, codeOf(l), (double*)nullptr, st);
       curBuf[l] = cb;
-      run(kResidualRestrict<TS, TS, TS>, gridOf(lv[l + 1].r), blk, lv[l], lv[l + 1].r, (const TS*)bL[l],
+      run(kResidualRestrict<TS, TS, TS>, restrictGrid(lv[l + 1].r), rblk, lv[l], lv[l + 1].r, (const TS*)bL[l],
           (const TS*)zl[cb], codeOf(l), bL[l + 1], (const CgState*)st);
     }
   }
@@ -621,9 +631,9 @@ const float* vcycleT(Multigrid* m, const float* r0, CgState* st, cudaStream_t s,
   {
     int l = L - 1;
     if (l == 0)
-      run(kCoarseSolve<float, float>, dim3(1), dim3(1024), lv[0], r0, z0[0], codeOf(0), (const CgState*)st);
+      run(kCoarseSolve<float, float>, dim3(1), dim3(kCoarseMax), lv[0], r0, z0[0], codeOf(0), (const CgState*)st);
     else
-      run(kCoarseSolve<TS, TS>, dim3(1), dim3(1024), lv[l], (const TS*)bL[l], zaL[l], codeOf(l), (const CgState*)st);
+      run(kCoarseSolve<TS, TS>, dim3(1), dim3(kCoarseMax), lv[l], (const TS*)bL[l], zaL[l], codeOf(l), (const CgState*)st);
     curBuf[l] = 0;
   }
   // upward sweep: prolongation fused into the first post-smoothing sweep
@@ -763,13 +773,20 @@ void mgRunCg(Multigrid* m, const Dim3i& cg, float sx, float sy, float sz, const 
     if (z != z0) throw CudaError("multigrid: V-cycle output buffer changed between iterations", HFG_ERR_STATE);
   };
   if (!*chunk) *chunk = capture(body);
+  // as many chunks as the last solve needed, less one, go out before the first
+  // convergence read
+  int batch = std::max(1, m->chunks - 1);
   for (;;) {
-    check(cudaGraphLaunch(*chunk, s), "cg chunk");
-    launches += m->chunkLaunches;
+    for (int k = 0; k < batch; ++k) {
+      check(cudaGraphLaunch(*chunk, s), "cg chunk");
+      launches += m->chunkLaunches;
+    }
     readBack(stHost, st, sizeof(CgState), s);
     check(cudaStreamSynchronize(s), "cg sync");
     if (stHost->done) break;
+    batch = 1;
   }
+  m->chunks = (stHost->iter + kChunk - 1) / kChunk;
 }
 
 }  // namespace hfg

@@ -8,6 +8,8 @@ import pytest
 import torch
 
 import hfgrid
+import oracle
+import scenes
 
 pytestmark = pytest.mark.gpu
 UNKNOWN = np.finfo(np.float32).max
@@ -104,3 +106,70 @@ def test_fluid_distance_field(cuda, res, layers):
     out = torch.empty(res[::-1], device=cuda)
     hfgrid.op_build_fluid_sdf(res, dev(dom), out, layers)
     assert np.array_equal(host(out), ref)
+
+
+# --- multigrid --------------------------------------------------------------------
+@pytest.mark.parametrize("res", [(15, 9, 11), (32, 16, 16), (33, 40, 18), (48, 25, 50), (64, 64, 30)])
+@pytest.mark.parametrize("half", [0, 1])
+def test_multigrid_level_splits(cuda, res, half):
+    """Ragged grids of two to five levels: the pressure of a converged multigrid
+    solve is the Jacobi solve's (both to 1e-6 of the right-hand side; the
+    system's smallest eigenvalue scales the difference up by < 100)."""
+    sc = scenes.Scene(res=res, seed=1, fluid_max=(0.7, 0.7, 1.0))
+    out = []
+    for opt in (dict(precond=2, mg_half=half), dict(precond=1)):
+        s = scenes.gpu_solver(sc, tol=1e-6, max_iter=4000, **opt)
+        s.update(2)
+        assert s.stats()["cg_converged"]
+        out.append((s.pressure().astype(np.float64), s.stats()["cg_iterations"]))
+    (pm, im), (pj, ij) = out
+    assert np.linalg.norm(pm - pj) < 2e-4 * np.linalg.norm(pj)
+    assert im <= ij
+
+
+# --- particle advection ------------------------------------------------------------
+@pytest.mark.parametrize("res", [(1, 1, 1), (2, 1, 3), (9, 8, 7)])
+@pytest.mark.parametrize("rk", [0, 1, 2])
+def test_substep_samples_at_and_beyond_the_grid(cuda, res, rk):
+    """Particles on cell centres, faces, edges of the grid and beyond it, one
+    step against the FP64 formula (a substep's rounding is a few 2**-24 of the
+    position: 1e-5 cells)."""
+    rng = np.random.default_rng(rk)
+    h = np.array((0.1, 0.12, 0.09))
+    o = np.array((0.25, -0.5, 1.0))
+    grid = np.stack(np.meshgrid(*[np.arange(-2, 2 * n + 3) / 2 for n in res], indexing="ij"), -1).reshape(-1, 3)
+    pos = (o + np.concatenate([grid, rng.random((200, 3)) * (np.array(res) + 2) - 1]) * h).astype(np.float32)
+    v = [rng.standard_normal(s).astype(np.float32) for s in oracle.face_shapes(res)]
+    dt = float(0.2 * h.min() / max(np.abs(a).max() for a in v))  # one substep
+
+    def sample(p):
+        out = np.empty_like(p)
+        for a in range(3):
+            f = v[a].astype(np.float64)
+            acc = np.zeros(len(p))
+            u = [(p[:, k] - o[k]) / h[k] - (0.0 if k == a else 0.5) for k in range(3)]
+            i = [np.floor(t).astype(int) for t in u]
+            w = [t - b for t, b in zip(u, i)]
+            for dz in (0, 1):
+                for dy in (0, 1):
+                    for dx in (0, 1):
+                        idx = [np.clip(i[k] + d, 0, f.shape[2 - k] - 1) for k, d in enumerate((dx, dy, dz))]
+                        acc += (np.where(dx, w[0], 1 - w[0]) * np.where(dy, w[1], 1 - w[1]) *
+                                np.where(dz, w[2], 1 - w[2])) * f[idx[2], idx[1], idx[0]]
+            out[:, a] = acc
+        return out
+
+    p = pos.astype(np.float64)
+    w0 = sample(p)
+    if rk == 0:
+        ref = p + dt * w0
+    elif rk == 1:
+        ref = p + dt * sample(p + 0.5 * dt * w0)
+    else:
+        w1 = sample(p + 0.5 * dt * w0)
+        ref = p + dt * (2 * w0 + 3 * w1 + 4 * sample(p + 0.75 * dt * w1)) / 9
+    ref = np.clip(ref, o, o + np.array(res) * h)
+    pd = dev(pos)
+    n = hfgrid.op_advect_particles(res, o, h, [dev(a) for a in v], pd, dt, 1.0, rk, clamp_mode=0)
+    assert n == 1
+    assert np.abs(host(pd) - ref).max() < 1e-5 * h.max() + 4 * 2.0 ** -24 * np.abs(ref).max()
