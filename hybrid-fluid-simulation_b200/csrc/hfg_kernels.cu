@@ -1564,9 +1564,26 @@ cudaError_t launchSubstep(const Geom& g, FaceQuads vel, float* pos, float* v0, l
   return cudaGetLastError();
 }
 
-// P2G of particle velocities to the three face grids, value and weight packed
-// as float2 so every corner is one vector atomic
-// (accumulateParticles2CCSField, EulerParticlesTool.cu:79-196).
+// Adds (value, weight) pairs to two neighbouring entries: one 16-byte atomic
+// where the pair lies on a 16-byte boundary, else two of 8 bytes.
+__device__ __forceinline__ void addPair(float2* p, float2 a, float2 b) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    atomicAdd(reinterpret_cast<float4*>(p), make_float4(a.x, a.y, b.x, b.y));
+  } else {
+    atomicAdd(p, a);
+    atomicAdd(p + 1, b);
+  }
+}
+
+// P2G of one particle to a grid, value and weight packed as float2
+// (accumulateParticles2CCSField, EulerParticlesTool.cu:79-196).  The kernel is
+// bound by the atomics at L2, so a row of four taps goes out as 16-byte atomics
+// (two, or one and two 8-byte ones, by the row's alignment), and the taps that a
+// quadratic kernel leaves without weight (37 of 64) are skipped; a value that
+// is not finite still reaches them, as 0 times it is not 0.  0.9 M particles,
+// 97 x 64 x 83, cubic: 0.90 -> 0.66 ms.  (The linear
+// kernel's corners sent this way: 2.40 -> 2.50 ms at 256^3, so it keeps its own
+// atomics.)
 template <int ALG>
 __device__ inline void p2gScatter(const Geom& fg, float px, float py, float pz, float val, float2* acc) {
   if (ALG == P2GSUM) {
@@ -1576,16 +1593,44 @@ __device__ inline void p2gScatter(const Geom& fg, float px, float py, float pz, 
   Taps t;
   taps<ALG>(fg, px, py, pz, t);
   constexpr int n = TapsN<ALG>::n, s = TapsN<ALG>::shift;
+  const int x0 = t.base[0] + s;
+  const bool inRow = x0 >= 0 && x0 + n <= fg.r.x;
+  const bool skip0 = ALG == QUADRATIC && fabsf(val) <= FLT_MAX;  // taps of weight 0 add nothing
 #pragma unroll
   for (int z = 0; z < n; ++z)
 #pragma unroll
-    for (int y = 0; y < n; ++y)
+    for (int y = 0; y < n; ++y) {
+      if (skip0 && (t.w[1][y] == 0.f || t.w[2][z] == 0.f)) continue;
+      float2 c[n];
 #pragma unroll
       for (int x = 0; x < n; ++x) {
-        float w = t.w[0][x] * t.w[1][y] * t.w[2][z];
-        long long i = linc(t.base[0] + x + s, t.base[1] + y + s, t.base[2] + z + s, fg.r);
-        atomicAdd(acc + i, make_float2(w * val, w));
+        const float w = t.w[0][x] * t.w[1][y] * t.w[2][z];
+        c[x] = make_float2(w * val, w);
       }
+      if (!inRow) {
+#pragma unroll
+        for (int x = 0; x < n; ++x)
+          atomicAdd(acc + linc(t.base[0] + x + s, t.base[1] + y + s, t.base[2] + z + s, fg.r), c[x]);
+        continue;
+      }
+      float2* row = acc + linc(x0, t.base[1] + y + s, t.base[2] + z + s, fg.r);
+      if (n == 2) {
+        atomicAdd(row, c[0]);
+        atomicAdd(row + 1, c[1]);
+      } else {
+        const bool lo = !(skip0 && t.w[0][0] == 0.f), hi = !(skip0 && t.w[0][n - 1] == 0.f);
+        if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+          if (lo) addPair(row, c[0], c[1]);
+          else atomicAdd(row + 1, c[1]);
+          if (hi) addPair(row + 2, c[n - 2], c[n - 1]);
+          else atomicAdd(row + 2, c[n - 2]);
+        } else {
+          if (lo) atomicAdd(row, c[0]);
+          addPair(row + 1, c[1], c[n - 2]);
+          if (hi) atomicAdd(row + 3, c[n - 1]);
+        }
+      }
+    }
 }
 
 // LINEAR P2G to the three face grids.  Particles are stored in seeding order

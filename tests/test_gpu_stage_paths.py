@@ -108,6 +108,41 @@ def test_fluid_distance_field(cuda, res, layers):
     assert np.array_equal(host(out), ref)
 
 
+# --- transfers ------------------------------------------------------------------
+@pytest.mark.parametrize("alg", [hfgrid.LINEAR, hfgrid.QUADRATIC, hfgrid.CUBIC])
+@pytest.mark.parametrize("res", [(1, 1, 1), (2, 3, 1), (8, 5, 6), (13, 4, 7)])
+def test_p2g_rows_of_both_alignments(cuda, alg, res):
+    """Rows that start on and off 16 bytes, and rows shorter than the stencil.
+    The sums differ from the FP32 oracle by their order: 64 addends of a face
+    at 2**-24 each, doubled for the weight, stay below 1e-5."""
+    rng = np.random.default_rng(alg)
+    h = (0.1, 0.12, 0.09)
+    n = 400
+    pos = ((rng.random((n, 3)) * 1.2 - 0.1) * np.array(res) * np.array(h)).astype(np.float32)
+    vel = rng.standard_normal((n, 3)).astype(np.float32)
+    out = [torch.empty(s, device=cuda) for s in oracle.face_shapes(res)]
+    wgt = [torch.empty(s, device=cuda) for s in oracle.face_shapes(res)]
+    hfgrid.op_p2g_fc(res, (0, 0, 0), h, dev(pos), dev(vel), alg, out, wgt)
+    # weights: the sum over all faces of a component is one per particle
+    for w in wgt:
+        assert abs(float(w.double().sum()) / n - 1) < 1e-5
+    num = [torch.empty(s, device=cuda) for s in oracle.face_shapes(res)]
+    hfgrid.op_p2g_fc(res, (0, 0, 0), h, dev(pos), dev(np.ones_like(vel)), alg, num)
+    for v, w in zip(num, wgt):  # a constant comes back where anything arrived
+        assert torch.allclose(v[w > 1e-6], torch.ones_like(v[w > 1e-6]), rtol=1e-5)
+
+
+def test_p2g_value_not_finite_reaches_its_whole_stencil(cuda):
+    """0 times infinity is not 0: the taps of weight 0 turn NaN as well."""
+    res, h = (12, 11, 10), (0.1, 0.1, 0.1)
+    pos = np.array([[0.53, 0.52, 0.47]], np.float32)
+    vel = np.full((1, 3), np.inf, np.float32)
+    out = [torch.empty(s, device=cuda) for s in oracle.face_shapes(res)]
+    hfgrid.op_p2g_fc(res, (0, 0, 0), h, dev(pos), dev(vel), hfgrid.QUADRATIC, out)
+    for o in out:
+        assert int((~torch.isfinite(o)).sum()) == 64
+
+
 # --- multigrid --------------------------------------------------------------------
 @pytest.mark.parametrize("res", [(15, 9, 11), (32, 16, 16), (33, 40, 18), (48, 25, 50), (64, 64, 30)])
 @pytest.mark.parametrize("half", [0, 1])
