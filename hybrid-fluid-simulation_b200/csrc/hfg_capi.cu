@@ -741,6 +741,15 @@ HFG_API int hfg_op_g2p_cc(const int res[3], const float origin[3], const float s
     return HFG_OK;
   });
 }
+static NormalizeFaces plainNormalize(const long long F[3], float2* const acc[3], float* const out[3]) {
+  NormalizeFaces f{};
+  for (int a = 0; a < 3; ++a) {
+    f.n[a] = F[a];
+    f.acc[a] = acc[a];
+    f.out[a] = out[a];
+  }
+  return f;
+}
 HFG_API int hfg_op_p2g_fc(const int res[3], const float origin[3], const float spacing[3], const float* pos,
                           const float* vel, long long n, int alg, float* vx, float* vy, float* vz, float* wx,
                           float* wy, float* wz, void* stream) {
@@ -751,14 +760,16 @@ HFG_API int hfg_op_p2g_fc(const int res[3], const float origin[3], const float s
     cudaStream_t s = st(stream);
     long long F[3] = {(long long)(res[0] + 1) * res[1] * res[2], (long long)res[0] * (res[1] + 1) * res[2],
                       (long long)res[0] * res[1] * (res[2] + 1)};
-    Scratch<float2> a0(F[0], s), a1(F[1], s), a2(F[2], s);
-    float2* acc[3] = {a0.p, a1.p, a2.p};
-    for (int a = 0; a < 3; ++a) check(cudaMemsetAsync(acc[a], 0, 8 * F[a], s), "memset");
+    long long at[3];
+    const long long total = faceAccumulators(F, at);
+    Scratch<float2> all(total, s);
+    float2* acc[3] = {all.p + at[0], all.p + at[1], all.p + at[2]};
+    check(cudaMemsetAsync(all.p, 0, 8 * total, s), "memset");
     check(launchP2GFace(g, alg, pos, vel, n, acc, s), "p2g");
     float* out[3] = {vx, vy, vz};
     float* w[3] = {wx, wy, wz};
+    check(launchNormalizeFaces(plainNormalize(F, acc, out), s), "normalize");
     for (int a = 0; a < 3; ++a) {
-      check(launchNormalize(F[a], acc[a], out[a], nullptr, 0.f, 0, 0.f, 0, s), "normalize");
       if (w[a]) check(cudaMemcpy2DAsync(w[a], 4, (const char*)acc[a] + 4, 8, 4, F[a], cudaMemcpyDeviceToDevice, s), "w");
     }
     check(cudaStreamSynchronize(s), "sync");
@@ -775,7 +786,7 @@ HFG_API int hfg_op_p2g_cc(const int res[3], const float origin[3], const float s
     Scratch<float2> acc(N, s);
     check(cudaMemsetAsync(acc.p, 0, 8 * N, s), "memset");
     check(launchP2GCell(g, alg, pos, val, 1, 0, n, acc.p, s), "p2g");
-    if (normalize) check(launchNormalize(N, acc.p, f, nullptr, 0.f, 0, 0.f, 0, s), "normalize");
+    if (normalize) check(launchNormalize(N, acc.p, f, s), "normalize");
     else check(cudaMemcpy2DAsync(f, 4, acc.p, 8, 4, N, cudaMemcpyDeviceToDevice, s), "copy");
     if (w) check(cudaMemcpy2DAsync(w, 4, (const char*)acc.p + 4, 8, 4, N, cudaMemcpyDeviceToDevice, s), "w");
     check(cudaStreamSynchronize(s), "sync");
@@ -1076,8 +1087,8 @@ HFG_API int hfg_op_p2g_fc_static(const int res[3], const float origin[3], const 
     check(launchP2GFace(g, alg, pos, vel, n, acc, s), "p2g");
     float* out[3] = {vx, vy, vz};
     float* w[3] = {wx, wy, wz};
+    check(launchNormalizeFaces(plainNormalize(F, acc, out), s), "normalize");
     for (int a = 0; a < 3; ++a) {
-      check(launchNormalize(F[a], acc[a], out[a], nullptr, 0.f, 0, 0.f, 0, s), "normalize");
       if (w[a]) check(cudaMemcpy2DAsync(w[a], 4, (const char*)acc[a] + 4, 8, 4, F[a], cudaMemcpyDeviceToDevice, s), "w");
     }
     check(cudaStreamSynchronize(s), "sync");

@@ -342,8 +342,33 @@ cudaError_t launchP2GFace(const Geom& g, int alg, const float* pos, const float*
                           cudaStream_t s);
 cudaError_t launchP2GCell(const Geom& g, int alg, const float* pos, const float* val, int span, int comp, long long P,
                           float2* acc, cudaStream_t s);
-cudaError_t launchNormalize(long long n, const float2* acc, float* out, float* copy, float add, int doAdd,
-                            float add2, int doAdd2, cudaStream_t s);
+cudaError_t launchNormalize(long long n, const float2* acc, float* out, cudaStream_t s);
+// P2G accumulators of three face grids of F[a] entries in one array: where each
+// starts (an even entry: 16 bytes) and the entries of all
+inline long long faceAccumulators(const long long F[3], long long at[3]) {
+  long long n = 0;
+  for (int a = 0; a < 3; ++a) {
+    at[a] = n;
+    n += (F[a] + 1) & ~1LL;
+  }
+  return n;
+}
+// the three face grids in one launch; copy (null: none) takes the value before
+// the additions
+struct NormalizeFaces {
+  long long n[3];
+  const float2* acc[3];
+  float *out[3], *copy[3];
+  float add[3], add2[3];
+  int doAdd, doAdd2;
+};
+cudaError_t launchNormalizeFaces(const NormalizeFaces& f, cudaStream_t s);
+// P2G of a vector and a scalar per particle to the cells (acc, weight cleared
+// by the caller) and the four normalised fields
+cudaError_t launchP2GCells(const Geom& g, int alg, const float* pos, const float* vec, const float* scalar, long long P,
+                           float4* acc, float* weight, cudaStream_t s);
+cudaError_t launchNormalizeCells(long long n, const float4* acc, const float* weight, float* const out[4],
+                                 cudaStream_t s);
 cudaError_t launchG2PFace(const Geom& g, int alg, ConstFaceField f, const float* pos, long long P, float* out,
                           cudaStream_t s);
 cudaError_t launchG2PCell(const Geom& g, int alg, const float* f, const float* pos, long long P, float* out, int span,

@@ -384,23 +384,35 @@ void GridSolver::forcesTerms(float gv[3], bool& doG, float ev[3], bool& doE) con
 
 void GridSolver::p2gFace(const float* vel, float* const out[3], float* const copy[3], const float add[3], bool doAdd,
                          const float add2[3], bool doAdd2) {
-  for (int a = 0; a < 3; ++a) {
-    acc_[a].alloc(F_[a], stream_);
-    check(cudaMemsetAsync(acc_[a].p, 0, acc_[a].bytes(), stream_), "memset");
-  }
-  float2* acc[3] = {acc_[0].p, acc_[1].p, acc_[2].p};
+  // the three accumulators in one array, cleared at once; each starts on 16 bytes
+  long long at[3];
+  const long long total = faceAccumulators(F_, at);
+  acc_.alloc(total, stream_);
+  check(cudaMemsetAsync(acc_.p, 0, acc_.bytes(), stream_), "memset");
+  float2* acc[3] = {acc_.p + at[0], acc_.p + at[1], acc_.p + at[2]};
   launched(launchP2GFace(g_, alg_, ppos_.p, vel, P_, acc, stream_), "p2g");
-  for (int a = 0; a < 3; ++a)
-    launched(launchNormalize(F_[a], acc_[a].p, out[a], copy ? copy[a] : nullptr, add ? add[a] : 0.f, doAdd,
-                             add2 ? add2[a] : 0.f, doAdd2, stream_),
-             "normalize");
+  NormalizeFaces nf{};
+  for (int a = 0; a < 3; ++a) {
+    nf.n[a] = F_[a];
+    nf.acc[a] = acc[a];
+    nf.out[a] = out[a];
+    nf.copy[a] = copy ? copy[a] : nullptr;
+    nf.add[a] = add ? add[a] : 0.f;
+    nf.add2[a] = add2 ? add2[a] : 0.f;
+  }
+  nf.doAdd = doAdd;
+  nf.doAdd2 = doAdd2;
+  launched(launchNormalizeFaces(nf, stream_), "normalize");
 }
 
-void GridSolver::p2gCell(const float* vals, int span, int comp, float* out) {
+// the particles' colour (pvector_) and domain (pscalar_) to the cells
+void GridSolver::p2gScalars(float* const out[4]) {
   cacc_.alloc(N_, stream_);
+  cweight_.alloc(N_, stream_);
   check(cudaMemsetAsync(cacc_.p, 0, cacc_.bytes(), stream_), "memset");
-  launched(launchP2GCell(g_, alg_, ppos_.p, vals, span, comp, P_, cacc_.p, stream_), "p2g cell");
-  launched(launchNormalize(N_, cacc_.p, out, nullptr, 0.f, 0, 0.f, 0, stream_), "normalize cell");
+  check(cudaMemsetAsync(cweight_.p, 0, cweight_.bytes(), stream_), "memset");
+  launched(launchP2GCells(g_, alg_, ppos_.p, pvector_.p, pscalar_.p, P_, cacc_.p, cweight_.p, stream_), "p2g cells");
+  launched(launchNormalizeCells(N_, cacc_.p, cweight_.p, out, stream_), "normalize cells");
 }
 
 // Corner tables of the advecting velocity (G2P and every substep sample read
@@ -582,12 +594,12 @@ void GridSolver::advectEnd() {
         launched(launchG2PCell(g_, alg_, color_[ci][a].p, ppos_.p, P_, pvector_.p, 3, a, stream_), "g2p colour");
       vFlag_ = true;
     }
-    for (int a = 0; a < 3; ++a) p2gCell(pvector_.p, 3, a, color_[ni][a].p);
     if (!sFlag_) {
       launched(launchG2PCell(g_, alg_, dom_[ci].p, ppos_.p, P_, pscalar_.p, 1, 0, stream_), "g2p domain");
       sFlag_ = true;
     }
-    p2gCell(pscalar_.p, 1, 0, dom_[ni].p);
+    float* out[4] = {color_[ni][0].p, color_[ni][1].p, color_[ni][2].p, dom_[ni].p};
+    p2gScalars(out);
   }
   stageEnd(1);
 }

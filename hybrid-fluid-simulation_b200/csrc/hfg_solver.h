@@ -175,7 +175,7 @@ class GridSolver {
   void advectParticles(const FaceQuads& v);
   void p2gFace(const float* vel, float* const out[3], float* const copy[3], const float add[3], bool doAdd,
                const float add2[3], bool doAdd2);
-  void p2gCell(const float* vals, int span, int comp, float* out);
+  void p2gScalars(float* const out[4]);
   void computePressure();
   void runCg();
   bool runCgResident(float sx, float sy, float sz, int pc);
@@ -235,7 +235,9 @@ class GridSolver {
   SubstepState* subHost_ = nullptr;  // pinned
   int subSlots_ = 4096;
   int cgChunks_ = 0;  // CG chunks the last Jacobi/identity solve needed
-  DArray<float2> acc_[3], cacc_;
+  DArray<float2> acc_;     // P2G accumulators of the three face grids (faceAccumulators)
+  DArray<float4> cacc_;    // and of the cells: colour and domain, their weight
+  DArray<float> cweight_;
   DArray<float4> quads_[3];  // corner tables of the advecting velocity (particle substeps)
   FaceQuads vq_{};           // their pointers during an advection
   DArray<uint16_t> dist_;

@@ -143,6 +143,31 @@ def test_p2g_value_not_finite_reaches_its_whole_stencil(cuda):
         assert int((~torch.isfinite(o)).sum()) == 64
 
 
+@pytest.mark.parametrize("alg", [hfgrid.LINEAR, hfgrid.QUADRATIC, hfgrid.CUBIC])
+def test_carried_scalars_match_the_operators(cuda, alg):
+    """One step's colour and domain against the transfers of the operators."""
+    sc = scenes.Scene(res=(20, 17, 13), seed=2)
+    s = scenes.gpu_solver(sc, advect_scalars=True, kind=hfgrid.ADV_PIC)
+    s.set_advection(hfgrid.ADV_PIC, hfgrid.RK3, alg, 1.0, 0.05)
+    s.seed_particles(4, 2)
+    rng = np.random.default_rng(1)
+    col = [rng.random(sc.res[::-1]).astype(np.float32) for _ in range(3)]
+    s.set_color_field(*col)
+    dom0 = s.fluid_domain_field()
+    p0, _ = s.particles()
+    s.update()
+    p1, _ = s.particles()
+    got = list(s.color_field()) + [s.fluid_domain_field()]
+    args = (sc.res, sc.origin, sc.spacing)
+    for f, g in zip(col + [dom0], got):
+        val = torch.empty(len(p0), device=cuda)
+        hfgrid.op_g2p_cc(*args, dev(f), dev(p0), alg, val)
+        ref = torch.empty(sc.res[::-1], device=cuda)
+        hfgrid.op_p2g_cc(*args, dev(p1), val, alg, ref)
+        # the order of the atomics: at most some 500 addends of one sign pattern
+        np.testing.assert_allclose(g, host(ref), rtol=2e-4, atol=1e-5 * np.abs(f).max())
+
+
 # --- multigrid --------------------------------------------------------------------
 @pytest.mark.parametrize("res", [(15, 9, 11), (32, 16, 16), (33, 40, 18), (48, 25, 50), (64, 64, 30)])
 @pytest.mark.parametrize("half", [0, 1])
