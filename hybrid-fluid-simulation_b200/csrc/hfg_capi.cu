@@ -66,12 +66,63 @@ Geom toGeom(const int r[3], const float* o, const float* h) {
 }
 cudaStream_t st(void* s) { return (cudaStream_t)s; }
 
+// The operators' scratch comes from a stream-ordered pool of this library's
+// own, one per device.  The device's default pool gives every freed byte back
+// to the driver at the next synchronisation, and each operator call ends in
+// one, so a call on its own paid for mapping its scratch again: 3.5 of the
+// 5.1 ms of a 160^3 particle advection.  This pool keeps up to kPoolKeep bytes
+// across synchronisations (more is given back as before), gives all of it back
+// when an allocation fails for lack of memory and is retried, and leaves the
+// default pool and its settings alone.  The driver orders reuse between
+// streams and threads, as for the default pool.
+constexpr unsigned long long kPoolKeep = 512ull << 20;
+constexpr int kPoolDevices = 64;
+cudaError_t scratchPool(cudaMemPool_t* pool) {
+  static std::mutex mu;
+  static cudaMemPool_t pools[kPoolDevices] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= kPoolDevices) return cudaDeviceGetDefaultMemPool(pool, dev);
+  std::lock_guard<std::mutex> lk(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    // the first call may come while its stream is being captured
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if ((e = cudaThreadExchangeStreamCaptureMode(&mode)) != cudaSuccess) return e;
+    cudaMemPool_t made = nullptr;
+    unsigned long long keep = kPoolKeep;
+    e = cudaMemPoolCreate(&made, &props);
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess && made) cudaMemPoolDestroy(made);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return e;
+    pools[dev] = made;
+  }
+  *pool = pools[dev];
+  return cudaSuccess;
+}
+
 // Stream-ordered scratch for the operator entry points.
 template <class T> struct Scratch {
   T* p = nullptr;
   cudaStream_t s;
   Scratch(size_t n, cudaStream_t s_) : s(s_) {
-    if (n && cudaMallocAsync((void**)&p, n * sizeof(T), s) != cudaSuccess) {
+    if (!n) return;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = scratchPool(&pool);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void**)&p, n * sizeof(T), pool, s);
+    if (e == cudaErrorMemoryAllocation) {
+      // what the pools hold unused, back to the driver, then once more
+      cudaGetLastError();
+      cudaMemPoolTrimTo(pool, 0);
+      e = cudaMallocFromPoolAsync((void**)&p, n * sizeof(T), pool, s);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
       p = nullptr;
       throw CudaError("cudaMallocAsync failed", HFG_ERR_NOMEM);
     }

@@ -2,6 +2,7 @@
 edges, one-cell axes, scan chunks, ragged multigrid levels, values that are not
 finite.
 """
+import threading
 
 import numpy as np
 import pytest
@@ -233,3 +234,41 @@ def test_substep_samples_at_and_beyond_the_grid(cuda, res, rk):
     n = hfgrid.op_advect_particles(res, o, h, [dev(a) for a in v], pd, dt, 1.0, rk, clamp_mode=0)
     assert n == 1
     assert np.abs(host(pd) - ref).max() < 1e-5 * h.max() + 4 * 2.0 ** -24 * np.abs(ref).max()
+
+
+# --- operator scratch -----------------------------------------------------------------
+def test_operators_on_several_threads_and_streams(cuda):
+    """The operators' scratch pool: the same results from four threads on
+    streams of their own, and at most its bound (512 MiB, and the driver's
+    granularity) stays with it afterwards."""
+    rng = np.random.default_rng(0)
+    res, h = (40, 36, 30), (1 / 40, 1 / 36, 1 / 30)
+    pos = dev(rng.random((20000, 3)).astype(np.float32))
+    vel = dev(rng.standard_normal((20000, 3)).astype(np.float32))
+    shapes = oracle.face_shapes(res)
+
+    def work(stream, outs):
+        with torch.cuda.stream(stream):
+            for _ in range(20):
+                hfgrid.op_p2g_fc(res, (0, 0, 0), h, pos, vel, hfgrid.LINEAR, outs)
+
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    runs = [(torch.cuda.Stream(), [torch.empty(s, device=cuda) for s in shapes]) for _ in range(4)]
+    threads = [threading.Thread(target=work, args=r) for r in runs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for _, outs in runs[1:]:
+        for a, b in zip(outs, runs[0][1]):
+            assert torch.allclose(a, b, rtol=1e-4, atol=1e-4)
+    big = (256, 256, 200)
+    v = [torch.zeros(s, device=cuda) for s in oracle.face_shapes(big)]
+    p = torch.rand((1000, 3), device=cuda)
+    hfgrid.op_advect_particles(big, (0, 0, 0), (1 / 256, 1 / 256, 1 / 200), v, p, 1 / 60)  # 0.9 GB of tables
+    del v
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    assert free0 - torch.cuda.mem_get_info()[0] < (512 + 256) << 20
