@@ -173,7 +173,7 @@ HFG_API int hfg_selftest_bounded_waits(int wait_ms, int* mbarrier_timed_out, int
     NEED(wait_ms > 0 && wait_ms <= 10000 && mbarrier_timed_out && grid_barrier_timed_out, "invalid arguments");
     DArray<unsigned> words;
     DArray<int> out;
-    words.alloc(3);
+    words.alloc(10);
     out.alloc(2);
     check(launchSelftestWaits((unsigned long long)wait_ms * 1000000ull, words.p, out.p, nullptr), "self-test");
     int h[2] = {-1, -1};
@@ -729,7 +729,7 @@ int extrapolateGrids(int ngrids, const Dim3i* rc, float* const* vals, int layers
   unsigned int words[4] = {0, 0, 0, 0};
   check(cudaMemcpyAsync(words, extrapBarWords(sc), sizeof(words), cudaMemcpyDeviceToHost, s), "read");
   check(cudaStreamSynchronize(s), "sync");
-  if (words[2] != 0u) return fail(HFG_ERR_TIMEOUT, "extrapolation: a grid barrier timed out");
+  if (words[kExtrapError] != 0u) return fail(HFG_ERR_TIMEOUT, "extrapolation: a grid barrier timed out");
   return HFG_OK;
 }
 }  // namespace

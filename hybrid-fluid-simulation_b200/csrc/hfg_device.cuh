@@ -665,36 +665,53 @@ __device__ __forceinline__ bool mbarWait(uint64_t* bar, unsigned parity, unsigne
     if (globalNs() > deadline) return false;
   return true;
 }
-// Grid barrier of a cooperative launch (generation counting).  The wait is
-// bounded: past the deadline, or once another block has given up, the error
-// word is set and false returned, and the caller stops.
-__device__ inline bool gridBarrier(unsigned* count, unsigned* gen, unsigned* err, unsigned nblocks) {
-  __shared__ int okS;
+// Orders this thread's memory accesses (and those its block's barrier has made
+// visible to it) before its later ones, GPU-wide.
+__device__ __forceinline__ void fenceGpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ unsigned ldRelaxed(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// The hardware barrier of a thread block cluster, in two halves; global writes
+// before the arrival are visible (through L2) to the cluster after the wait.
+__device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+// Grid barrier of a cooperative launch, in two halves so that work which needs
+// nothing of the other blocks can run between them.  Every block has a
+// mailbox with a word for each block (mail: nblocks^2 words, zeroed before the
+// launch): block b stores the epoch (1, 2, ...) into its word of all the
+// mailboxes and polls its own, so a barrier is one store and one load deep
+// and no line is polled by more than one SM.  A word may already hold the next
+// epoch.  The wait is bounded: past the deadline, or once another block has
+// given up, the error word is set and false returned, and the caller stops.
+__device__ inline void gridArrive(unsigned* mail, unsigned epoch, unsigned nblocks) {
   __syncthreads();
-  if (flatTid() == 0) {
-    int ok = 1;
-    const unsigned g = ldAcquire(gen);
-    __threadfence();  // this block's writes before its arrival
-    if (atomicAdd(count, 1u) == nblocks - 1) {
-      atomicExch(count, 0u);
-      __threadfence();
-      atomicAdd(gen, 1u);
-    } else {
-      const unsigned long long deadline = globalNs() + 1000000000ull;  // 1 s
-      while (ldAcquire(gen) == g) {
-        if (ldAcquire(err) != 0u || globalNs() > deadline) {
-          atomicExch(err, 1u);
-          ok = 0;
-          break;
-        }
-        __nanosleep(32);
+  const unsigned tid = flatTid(), threads = blockThreads(), me = flatBlock();
+  if (tid < nblocks) fenceGpu();  // this block's writes before its arrival
+  for (unsigned j = tid; j < nblocks; j += threads)
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(mail + (size_t)j * nblocks + me), "r"(epoch) : "memory");
+}
+__device__ inline bool gridWait(const unsigned* mail, unsigned epoch, unsigned* err, unsigned nblocks) {
+  const unsigned tid = flatTid(), threads = blockThreads(), me = flatBlock();
+  bool fail = false;
+  for (unsigned j = tid; j < nblocks && !fail; j += threads) {
+    unsigned long long deadline = 0;
+    for (int spin = 0; (int)(ldRelaxed(mail + (size_t)me * nblocks + j) - epoch) < 0; ++spin) {
+      if ((spin & 63) != 63) continue;
+      const unsigned long long now = globalNs();
+      if (deadline == 0) deadline = now + 1000000000ull;  // 1 s
+      if (now > deadline || ldRelaxed(err) != 0u) {
+        atomicExch(err, 1u);
+        fail = true;
+        break;
       }
     }
-    __threadfence();
-    okS = ok;
   }
-  __syncthreads();
-  return okS != 0;
+  if (tid < nblocks) fenceGpu();
+  return __syncthreads_or(fail) == 0;
 }
 
 // Asks L2 for the line holding *p ahead of its load (no register is held
@@ -724,5 +741,25 @@ inline cudaError_t launchPdl(void (*kernel)(KP...), dim3 grid, dim3 block, cudaS
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
+
+// One cluster of `size` blocks as the whole grid.
+template <class... KP, class... A>
+inline cudaError_t launchCluster(void (*kernel)(KP...), int size, int threads, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(size);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+// The largest cluster (16 blocks, else 8) of this kernel that the device can
+// hold, 0 if neither; asked once per kernel and device.  Lets the kernel be launched so.
+cudaError_t clusterSize(const void* kernel, int threads, size_t smem, int* size);
 
 }  // namespace hfg

@@ -9,6 +9,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstdio>
+#include <map>
 #include <mutex>
 
 #include "hfg_kernels.h"
@@ -49,6 +50,45 @@ __device__ inline void cellCoord(long long c, const Dim3i& r, int& x, int& y, in
 }
 
 }  // namespace
+
+cudaError_t clusterSize(const void* kernel, int threads, size_t smem, int* size) {
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, int> known;  // by kernel and device
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = known.find({kernel, dev});
+  if (it != known.end()) {
+    *size = it->second;
+    return cudaSuccess;
+  }
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess && smem > 0)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  *size = 0;
+  for (int n : {16, 8}) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(n);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = n;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) {
+      *size = n;
+      break;
+    }
+    cudaGetLastError();
+  }
+  known[{kernel, dev}] = *size;
+  return cudaSuccess;
+}
 
 int numSMs() {
   if (g_numSMs == 0) {
@@ -326,27 +366,34 @@ cudaError_t launchGradient(const Geom& g, float gx, float gy, float gz, const ui
 
 constexpr uint16_t kFar = 0xFFFF;
 
-__global__ void kDistInit(long long n, const float* __restrict__ v, uint16_t* __restrict__ d) {
-  HFG_FOR(i, n) d[i] = (v[i] == kUnknown) ? kFar : 0;
-}
-
 __device__ inline uint16_t satInc(uint16_t a) { return a >= kFar - 1 ? kFar : (uint16_t)(a + 1); }
 
-// 1-D pass along x: one warp per row, 32 entries at a time.  The forward
-// sweep f[i] = min(d[i], f[i-1] + 1) is a warp prefix-min of d[j] - j plus the
-// carry from the previous chunk; the backward sweep mirrors it.
-__global__ void kDistRows(Dim3i r, uint16_t* __restrict__ d) {
+// The grids of one extrapolation: up to three (one per blockIdx.y), an unused
+// one with no entries.
+struct ExtrapGrids {
+  Dim3i r[3];
+  float* v[3];
+  unsigned off[3];  // first entry of each grid in the joint numbering
+};
+
+// First distances and the 1-D pass along x: one warp per row, 32 entries at a
+// time.  The forward sweep f[i] = min(d[i], f[i-1] + 1), d = 0 at known
+// entries, is a warp prefix-min of d[j] - j plus the carry from the previous
+// chunk; the backward sweep mirrors it.
+__global__ void kDistRows(const __grid_constant__ ExtrapGrids g, uint16_t* __restrict__ dist) {
   constexpr int BIG = 1 << 20;
+  const Dim3i r = g.r[blockIdx.y];
+  const float* __restrict__ val = g.v[blockIdx.y];
+  uint16_t* __restrict__ d = dist + g.off[blockIdx.y];
   const int lane = threadIdx.x & 31;
-  long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  long long rows = (long long)r.y * r.z;
-  for (long long row = wid; row < rows; row += nw) {
-    uint16_t* q = d + row * r.x;
+  const int rows = r.y * r.z, nw = (int)(gridDim.x * blockDim.x) >> 5;
+  for (int row = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += nw) {
+    uint16_t* q = d + (size_t)row * r.x;
+    const float* p = val + (size_t)row * r.x;
     int carry = BIG;
     for (int s0 = 0; s0 < r.x; s0 += 32) {
       int i = s0 + lane;
-      int v = i < r.x ? (q[i] == kFar ? BIG : (int)q[i]) : BIG;
+      int v = i < r.x && p[i] != kUnknown ? 0 : BIG;
       int a = v - lane;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -368,42 +415,44 @@ __global__ void kDistRows(Dim3i r, uint16_t* __restrict__ d) {
         int t = __shfl_down_sync(0xffffffffu, b, o);
         if (lane + o < 32) b = min(b, t);
       }
-      int g = min(b - lane, carry + (32 - lane));
-      if (i < r.x) q[i] = (uint16_t)min(g, (int)kFar);
-      carry = __shfl_sync(0xffffffffu, g, 0);
+      int gm = min(b - lane, carry + (32 - lane));
+      if (i < r.x) q[i] = (uint16_t)min(gm, (int)kFar);
+      carry = __shfl_sync(0xffffffffu, gm, 0);
     }
   }
 }
 
-// 1-D pass along y or z: threads walk columns, coalesced across x.
-__global__ void kDistCols(Dim3i r, int axis, uint16_t* __restrict__ d) {
-  long long stride = axis == 1 ? r.x : (long long)r.x * r.y;
-  int len = axis == 1 ? r.y : r.z;
-  long long lines = axis == 1 ? (long long)r.x * r.z : (long long)r.x * r.y;
-  HFG_FOR(l, lines) {
-    long long base;
+// 1-D pass along y or z: threads walk columns, coalesced across x.  Columns
+// in batches of B: the B loads of a batch are in flight together, then the
+// batch is relaxed in order.  Both axes of three
+// 256^3 grids, with batches of 16 and one launch per axis: 283 -> 179 us.
+__global__ void kDistCols(const __grid_constant__ ExtrapGrids g, int axis, uint16_t* __restrict__ dist) {
+  const Dim3i r = g.r[blockIdx.y];
+  uint16_t* __restrict__ d = dist + g.off[blockIdx.y];
+  const unsigned nx = (unsigned)r.x, plane = nx * (unsigned)r.y;
+  const unsigned stride = axis == 1 ? nx : plane;
+  const int len = axis == 1 ? r.y : r.z;
+  const unsigned lines = axis == 1 ? nx * (unsigned)r.z : plane;
+  for (unsigned l = blockIdx.x * blockDim.x + threadIdx.x; l < lines; l += gridDim.x * blockDim.x) {
+    unsigned base = l;
     if (axis == 1) {
-      long long x = l % r.x, z = l / r.x;
-      base = z * r.x * (long long)r.y + x;
-    } else {
-      base = l;
+      const unsigned z = l / nx;
+      base = z * plane + (l - z * nx);
     }
-    // the column in batches of B: the B loads of a batch are in flight
-    // together, then the batch is relaxed in order
-    constexpr int B = 8;
+    constexpr int B = 16;
     uint16_t* col = d + base;
     uint16_t prev = kFar;
     for (int i0 = 0; i0 < len; i0 += B) {
       uint16_t v[B];
 #pragma unroll
-      for (int k = 0; k < B; ++k) v[k] = i0 + k < len ? col[(long long)(i0 + k) * stride] : kFar;
+      for (int k = 0; k < B; ++k) v[k] = i0 + k < len ? col[(unsigned)(i0 + k) * stride] : kFar;
 #pragma unroll
       for (int k = 0; k < B; ++k) {
         if (i0 + k < len) {
           const uint16_t cand = satInc(prev);
           if (cand < v[k]) {
             v[k] = cand;
-            col[(long long)(i0 + k) * stride] = cand;
+            col[(unsigned)(i0 + k) * stride] = cand;
           }
           prev = v[k];
         }
@@ -413,14 +462,14 @@ __global__ void kDistCols(Dim3i r, int axis, uint16_t* __restrict__ d) {
     for (int i0 = len - 1; i0 >= 0; i0 -= B) {
       uint16_t v[B];
 #pragma unroll
-      for (int k = 0; k < B; ++k) v[k] = i0 - k >= 0 ? col[(long long)(i0 - k) * stride] : kFar;
+      for (int k = 0; k < B; ++k) v[k] = i0 - k >= 0 ? col[(unsigned)(i0 - k) * stride] : kFar;
 #pragma unroll
       for (int k = 0; k < B; ++k) {
         if (i0 - k >= 0) {
           const uint16_t cand = satInc(prev);
           if (cand < v[k]) {
             v[k] = cand;
-            col[(long long)(i0 - k) * stride] = cand;
+            col[(unsigned)(i0 - k) * stride] = cand;
           }
           prev = v[k];
         }
@@ -430,25 +479,49 @@ __global__ void kDistCols(Dim3i r, int axis, uint16_t* __restrict__ d) {
 }
 
 // Histogram of layers 1..nums-1 (layers >= nums stay UNKNOWN).
-__global__ void kDistHist(long long n, const uint16_t* __restrict__ d, int nums, unsigned int* __restrict__ hist) {
+__global__ void kDistHist(unsigned n, const uint16_t* __restrict__ d, int nums, unsigned int* __restrict__ hist) {
   __shared__ unsigned int sh[kMaxLayers + 1];
   for (int i = threadIdx.x; i <= kMaxLayers; i += blockDim.x) sh[i] = 0;
   __syncthreads();
-  HFG_FOR(i, n) {
-    uint16_t v = d[i];
-    if (v >= 1 && v < nums) atomicAdd(&sh[v], 1u);
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const unsigned v = d[i];
+    if (v >= 1 && (int)v < nums) atomicAdd(&sh[v], 1u);
   }
   __syncthreads();
   for (int i = threadIdx.x; i <= kMaxLayers; i += blockDim.x)
     if (sh[i]) atomicAdd(hist + i, sh[i]);
 }
 
-__global__ void kExclusiveScanSmall(const unsigned int* __restrict__ hist, unsigned int* __restrict__ off,
-                                    unsigned int* __restrict__ cursor, int n) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    unsigned int s = 0;
-    for (int i = 0; i < n; ++i) { off[i] = s; cursor[i] = s; s += hist[i]; }
-    off[n] = s;
+// Exclusive scan of at most 1024 counts by one block.
+__global__ void __launch_bounds__(1024) kExclusiveScanSmall(const unsigned int* __restrict__ hist,
+                                                            unsigned int* __restrict__ off,
+                                                            unsigned int* __restrict__ cursor, int n) {
+  __shared__ unsigned int tot[32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const unsigned mine = t < n ? hist[t] : 0u;
+  unsigned inc = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  if (lane == 31) tot[w] = inc;
+  __syncthreads();
+  if (w == 0) {
+    unsigned v = tot[lane], vi = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned u = __shfl_up_sync(0xffffffffu, vi, o);
+      if (lane >= o) vi += u;
+    }
+    tot[lane] = vi - v;
+  }
+  __syncthreads();
+  const unsigned ex = tot[w] + inc - mine;
+  if (t < n) {
+    off[t] = ex;
+    cursor[t] = ex;
+    if (t == n - 1) off[n] = ex + mine;
   }
 }
 
@@ -467,71 +540,111 @@ __device__ __forceinline__ void extrapNeighbours(const Dim3i& r, unsigned i, uns
 }
 
 // Bucket the entries by layer: a block counts its chunk per layer in shared
-// memory, reserves one global range per (block, layer) and hands out slots
-// with shared-memory atomics.  Each entry also gets the mask of its
-// neighbours in earlier layers, so that the layer pass reads no distances.
-constexpr int kScatterChunk = 4096;
-__global__ void kDistScatter(Dim3i r, long long base, const uint16_t* __restrict__ d, int nums,
-                             unsigned int* __restrict__ cursor, unsigned int* __restrict__ list,
-                             uint8_t* __restrict__ mask) {
-  const long long n = r.size();
+// memory (the count before an entry is its rank), reserves one global range
+// per (block, layer) and writes the entries to their slots.  Only the bins
+// between the chunk's lowest and highest layer are touched: neighbouring
+// entries have neighbouring layers.  Each entry also gets the mask of its
+// neighbours in earlier layers, so that the layer pass reads no distances
+// (reading them there instead cost a layer 1.5 us: three loads deep).
+// Against clearing and reserving all 1001 bins with a second shared atomic
+// per entry: 555 -> 489 us (256^3, three grids).
+constexpr int kScatterThreads = 512, kScatterPer = 8, kScatterChunk = kScatterThreads * kScatterPer;
+__global__ void __launch_bounds__(kScatterThreads)
+    kDistScatter(const __grid_constant__ ExtrapGrids g, const uint16_t* __restrict__ dist, int nums, unsigned int* __restrict__ cursor,
+                 unsigned int* __restrict__ list, uint8_t* __restrict__ mask) {
+  const Dim3i r = g.r[blockIdx.y];
+  const unsigned base = g.off[blockIdx.y], n = (unsigned)r.size();
+  const uint16_t* __restrict__ d = dist + base;
   __shared__ unsigned int cnt[kMaxLayers + 1], start[kMaxLayers + 1];
-  for (long long c0 = (long long)blockIdx.x * kScatterChunk; c0 < n; c0 += (long long)gridDim.x * kScatterChunk) {
-    long long c1 = c0 + kScatterChunk < n ? c0 + kScatterChunk : n;
-    for (int i = threadIdx.x; i <= kMaxLayers; i += blockDim.x) cnt[i] = 0;
+  __shared__ int lo, hi;
+  for (unsigned c0 = blockIdx.x * kScatterChunk; c0 < n; c0 += gridDim.x * kScatterChunk) {
+    if (threadIdx.x == 0) {
+      lo = kMaxLayers + 1;
+      hi = 0;
+    }
+    unsigned v[kScatterPer], rank[kScatterPer];
+    unsigned mn = kMaxLayers + 1, mx = 0;
+#pragma unroll
+    for (int k = 0; k < kScatterPer; ++k) {
+      const unsigned i = c0 + k * kScatterThreads + threadIdx.x;
+      const unsigned dv = i < n ? d[i] : 0u;
+      v[k] = dv >= 1 && (int)dv < nums ? dv : 0u;
+      if (v[k]) {
+        mn = min(mn, dv);
+        mx = max(mx, dv);
+      }
+    }
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    mx = __reduce_max_sync(0xffffffffu, mx);
     __syncthreads();
-    for (long long i = c0 + threadIdx.x; i < c1; i += blockDim.x) {
-      unsigned int v = d[i];
-      if (v >= 1 && (int)v < nums) atomicAdd(&cnt[v], 1u);
+    if ((threadIdx.x & 31) == 0 && mx > 0) {
+      atomicMin(&lo, (int)mn);
+      atomicMax(&hi, (int)mx);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i <= kMaxLayers; i += blockDim.x) {
-      unsigned int k = cnt[i];
-      start[i] = k ? atomicAdd(cursor + i, k) : 0u;
-      cnt[i] = 0;
-    }
+    const int l0 = lo, l1 = hi;
+    for (int i = l0 + threadIdx.x; i <= l1; i += kScatterThreads) cnt[i] = 0;
     __syncthreads();
-    for (long long i = c0 + threadIdx.x; i < c1; i += blockDim.x) {
-      unsigned int v = d[i];
-      if (v >= 1 && (int)v < nums) {
+#pragma unroll
+    for (int k = 0; k < kScatterPer; ++k)
+      if (v[k]) rank[k] = atomicAdd(&cnt[v[k]], 1u);
+    __syncthreads();
+    for (int i = l0 + threadIdx.x; i <= l1; i += kScatterThreads) start[i] = cnt[i] ? atomicAdd(cursor + i, cnt[i]) : 0u;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kScatterPer; ++k) {
+      if (v[k]) {
+        const unsigned i = c0 + k * kScatterThreads + threadIdx.x;
         unsigned nb[6];
-        extrapNeighbours(r, (unsigned)i, nb);
+        extrapNeighbours(r, i, nb);
         unsigned m = 0;
 #pragma unroll
-        for (int q = 0; q < 6; ++q) m |= (unsigned)(d[nb[q]] < v) << q;
-        const unsigned slot = start[v] + atomicAdd(&cnt[v], 1u);
-        list[slot] = (unsigned int)(base + i);
+        for (int q = 0; q < 6; ++q) m |= (unsigned)(d[nb[q]] < v[k]) << q;
+        const unsigned slot = start[v[k]] + rank[k];
+        list[slot] = base + i;
         mask[slot] = (uint8_t)m;
       }
     }
-    __syncthreads();
   }
 }
+
+namespace {
+ExtrapGrids extrapGrids(const Dim3i rc[3], float* const vals[3], const long long off[3]) {
+  ExtrapGrids g;
+  for (int a = 0; a < 3; ++a) {
+    g.r[a] = rc[a];
+    g.v[a] = vals[a];
+    g.off[a] = (unsigned)off[a];
+  }
+  return g;
+}
+}  // namespace
 
 cudaError_t launchExtrapDistance(const Dim3i rc[3], float* const vals[3], long long off[3], int nums,
                                  ExtrapScratch sc, cudaStream_t s) {
   if (nums > kMaxLayers) nums = kMaxLayers;
+  const ExtrapGrids g = extrapGrids(rc, vals, off);
+  long long rows = 1, colsY = 1, colsZ = 1, most = 1, total = 0;
+  int grids = 0;
   for (int a = 0; a < 3; ++a) {
-    long long n = rc[a].size();
-    uint16_t* d = sc.dist + off[a];
-    kDistInit<<<gridFor(n), kThreads, 0, s>>>(n, vals[a], d);
-    kDistRows<<<gridFor((long long)rc[a].y * rc[a].z * 32), kThreads, 0, s>>>(rc[a], d);
-    kDistCols<<<gridFor((long long)rc[a].x * rc[a].z), kThreads, 0, s>>>(rc[a], 1, d);
-    kDistCols<<<gridFor((long long)rc[a].x * rc[a].y), kThreads, 0, s>>>(rc[a], 2, d);
+    if (rc[a].size() > 0) grids = a + 1;
+    rows = std::max(rows, (long long)rc[a].y * rc[a].z * 32);
+    colsY = std::max(colsY, (long long)rc[a].x * rc[a].z);
+    colsZ = std::max(colsZ, (long long)rc[a].x * rc[a].y);
+    most = std::max(most, rc[a].size());
+    total += rc[a].size();
   }
+  kDistRows<<<dim3(gridFor(rows), grids), kThreads, 0, s>>>(g, sc.dist);
+  kDistCols<<<dim3(gridFor(colsY, 128), grids), 128, 0, s>>>(g, 1, sc.dist);
+  kDistCols<<<dim3(gridFor(colsZ, 128), grids), 128, 0, s>>>(g, 2, sc.dist);
   cudaError_t e = cudaMemsetAsync(sc.hist, 0, sizeof(unsigned int) * kExtrapHistWords, s);
   if (e != cudaSuccess) return e;
-  for (int a = 0; a < 3; ++a) {
-    long long n = rc[a].size();
-    kDistHist<<<gridFor(n, kThreads, 4), kThreads, 0, s>>>(n, sc.dist + off[a], nums, sc.hist);
-  }
-  kExclusiveScanSmall<<<1, 1, 0, s>>>(sc.hist, sc.offsets, sc.cursor, kMaxLayers + 1);
-  for (int a = 0; a < 3; ++a) {
-    long long n = rc[a].size();
-    int blocks = (int)std::min<long long>((n + kScatterChunk - 1) / kScatterChunk, (long long)numSMs() * 8);
-    if (blocks < 1) blocks = 1;
-    kDistScatter<<<blocks, kThreads, 0, s>>>(rc[a], off[a], sc.dist + off[a], nums, sc.cursor, sc.list, sc.mask);
-  }
+  // every block adds its bins to the global ones: few blocks on small grids
+  kDistHist<<<gridFor(total, kThreads, total > 8000000 ? 16 : 4), kThreads, 0, s>>>((unsigned)total, sc.dist, nums, sc.hist);
+  kExclusiveScanSmall<<<1, 1024, 0, s>>>(sc.hist, sc.offsets, sc.cursor, kMaxLayers + 1);
+  const int blocks =
+      (int)std::min<long long>((most + kScatterChunk - 1) / kScatterChunk, (long long)numSMs() * 8);
+  kDistScatter<<<dim3(blocks, grids), kScatterThreads, 0, s>>>(g, sc.dist, nums, sc.cursor, sc.list, sc.mask);
   return cudaGetLastError();
 }
 
@@ -541,72 +654,110 @@ cudaError_t launchExtrapDistance(const Dim3i rc[3], float* const vals[3], long l
 // The values of earlier layers were written by other blocks of the same
 // launch, so they are read from L2 (ld.cg), never from a stale L1 line.
 // 32-bit index arithmetic: every face grid holds fewer than 2^31 entries.
-__device__ __forceinline__ void extrapEntry(const Dim3i& r0, const Dim3i& r1, const Dim3i& r2, float* v0, float* v1,
-                                            float* v2, unsigned off1, unsigned off2, unsigned id, unsigned m) {
-  const int a = id >= off2 ? 2 : (id >= off1 ? 1 : 0);
-  const unsigned base = a == 2 ? off2 : (a == 1 ? off1 : 0u);
-  const unsigned i = id - base;
-  const Dim3i r = a == 2 ? r2 : (a == 1 ? r1 : r0);
-  float* v = a == 2 ? v2 : (a == 1 ? v1 : v0);
-  unsigned nb[6];
-  extrapNeighbours(r, i, nb);
+struct ExtrapEntry {
+  float* v = nullptr;  // null: no entry
+  unsigned i, nb[6], m;
+};
+__device__ __forceinline__ ExtrapEntry extrapFetch(const ExtrapGrids& g, const unsigned* __restrict__ list,
+                                                   const uint8_t* __restrict__ mask, unsigned k, unsigned end) {
+  ExtrapEntry e;
+  if (k < end) {
+    const unsigned id = __ldg(list + k);
+    e.m = __ldg(mask + k);
+    const int a = id >= g.off[2] ? 2 : (id >= g.off[1] ? 1 : 0);
+    const Dim3i r = a == 2 ? g.r[2] : (a == 1 ? g.r[1] : g.r[0]);
+    e.v = a == 2 ? g.v[2] : (a == 1 ? g.v[1] : g.v[0]);
+    e.i = id - (a == 2 ? g.off[2] : (a == 1 ? g.off[1] : 0u));
+    extrapNeighbours(r, e.i, e.nb);
+  }
+  return e;
+}
+__device__ __forceinline__ void extrapFill(const ExtrapEntry& e) {
+  if (!e.v) return;
+  float w[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) w[q] = (e.m >> q) & 1u ? __ldcg(e.v + e.nb[q]) : 0.f;
   float acc = 0.f, cnt = 0.f;
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
-    if ((m >> q) & 1u) {
-      acc = __fadd_rn(acc, __ldcg(v + nb[q]));
+    if ((e.m >> q) & 1u) {
+      acc = __fadd_rn(acc, w[q]);
       cnt = __fadd_rn(cnt, 1.f);
     }
   }
   if (cnt != 0.f) acc = __fdiv_rn(acc, cnt);
-  v[i] = acc;
+  __stcg(e.v + e.i, acc);
 }
 
-// Block shape of the layer pass: 512 threads, at most two blocks per SM
-// (fewer, larger blocks than 256 x 4 meet at the grid barriers sooner).
-constexpr int kExtrapThreads = 512, kExtrapPerSM = 2;
+// Block shape of the layer pass: 1024 threads, at most one block per SM, as few
+// arrivals as possible at the barriers.
+constexpr int kExtrapThreads = 1024;
 
-// Layers 1 .. nums-1, persistent: a layer with more than kExtrapSmallLayer
-// faces is spread over the grid; a run of smaller consecutive layers is filled
-// by block 0 alone with block barriers between them.  Every block walks the
-// same layer bounds (sc.offsets), so all meet at the same grid barriers.
-// barWords: count, generation, error, deepest layer filled.
-__global__ void __launch_bounds__(kExtrapThreads)
-    kExtrapLayers(Dim3i r0, Dim3i r1, Dim3i r2, float* v0, float* v1, float* v2, unsigned off1, unsigned off2,
-                  const uint8_t* __restrict__ mask, const unsigned int* __restrict__ list,
-                  const unsigned int* __restrict__ offsets, int nums, unsigned* barWords) {
-  unsigned* count = barWords;
-  unsigned* gen = barWords + 1;
-  unsigned* err = barWords + 2;
-  const unsigned stride = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
+// Layers 1 .. nums-1, persistent: a layer of some size is spread over the
+// blocks; a run of smaller consecutive layers is filled by block 0 alone with
+// block barriers between them.  Every block walks the same layer bounds
+// (sc.offsets), so all meet at the same barriers.  A layer is bound by latency:
+// its faces are one or a few to a thread, and each step is neighbour loads, a
+// store and a barrier.  So a thread's first face of the next phase is fetched
+// and decoded while the barrier is on its way, and the loads of the neighbours
+// that count are in flight together.
+// CLUSTER: the blocks are one thread block cluster and meet at its hardware
+// barrier; otherwise they are a cooperative grid and meet through mailboxes.
+// barWords: kExtrapError, kExtrapDepth, then the mailboxes.
+template <bool CLUSTER>
+__global__ void __launch_bounds__(kExtrapThreads, 1)
+    kExtrapLayers(const __grid_constant__ ExtrapGrids g, const uint8_t* __restrict__ mask,
+                  const unsigned int* __restrict__ list, const unsigned int* __restrict__ offsets, int nums,
+                  unsigned* barWords) {
+  // a layer of at most this many faces is filled by block 0
+  constexpr unsigned kSmall = CLUSTER ? kExtrapThreads : kExtrapSmallLayer;
+  __shared__ unsigned offS[kMaxLayers + 2];
+  for (int i = threadIdx.x; i < kMaxLayers + 2; i += kExtrapThreads) offS[i] = __ldg(offsets + i);
+  __syncthreads();
+  unsigned* mail = barWords + kExtrapSlots;
+  const unsigned nblk = gridDim.x, stride = nblk * kExtrapThreads;
+  const unsigned gtid = blockIdx.x * kExtrapThreads + threadIdx.x;
+  auto size = [&](int d) -> unsigned {  // faces of layer d, 0 past the last layer
+    return d < nums && d <= kMaxLayers ? offS[d + 1] - offS[d] : 0u;
+  };
+  auto fetch = [&](int d, unsigned k) -> ExtrapEntry {  // k-th face of layer d
+    return extrapFetch(g, list, mask, offS[d] + k, offS[d] + size(d));
+  };
+  // this thread's first face of a phase that starts at layer d
+  auto firstOf = [&](int d) -> ExtrapEntry {
+    if (size(d) == 0) return ExtrapEntry{};
+    return fetch(d, size(d) > kSmall ? gtid : (blockIdx.x == 0 ? threadIdx.x : size(d)));
+  };
+  unsigned epoch = 0;
   int d = 1;
-  while (d < nums && d <= kMaxLayers) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) barWords[3] = (unsigned)(d - 1);
-    const unsigned b = __ldg(offsets + d), e = __ldg(offsets + d + 1);
-    if (e <= b) break;
-    if (e - b > kExtrapSmallLayer) {
-      for (unsigned k = b + gtid; k < e; k += stride) extrapEntry(r0, r1, r2, v0, v1, v2, off1, off2, list[k], mask[k]);
+  ExtrapEntry e = firstOf(d);
+  while (size(d) > 0) {
+    if (size(d) > kSmall) {
+      extrapFill(e);
+      for (unsigned k = gtid + stride; k < size(d); k += stride) extrapFill(fetch(d, k));
       ++d;
     } else {
       int last = d;
-      while (last + 1 < nums && last + 1 <= kMaxLayers) {
-        const unsigned nb = __ldg(offsets + last + 1), ne = __ldg(offsets + last + 2);
-        if (ne <= nb || ne - nb > kExtrapSmallLayer) break;
-        ++last;
-      }
+      while (size(last + 1) > 0 && size(last + 1) <= kSmall) ++last;
       if (blockIdx.x == 0) {
         for (int l = d; l <= last; ++l) {
-          const unsigned lb = __ldg(offsets + l), le = __ldg(offsets + l + 1);
-          for (unsigned k = lb + threadIdx.x; k < le; k += blockDim.x)
-            extrapEntry(r0, r1, r2, v0, v1, v2, off1, off2, list[k], mask[k]);
+          extrapFill(e);
+          for (unsigned k = threadIdx.x + kExtrapThreads; k < size(l); k += kExtrapThreads) extrapFill(fetch(l, k));
+          if (l < last) e = fetch(l + 1, threadIdx.x);
           __syncthreads();
         }
       }
       d = last + 1;
     }
-    if (gridDim.x > 1 && !gridBarrier(count, gen, err, gridDim.x)) return;
+    if (size(d) == 0) break;
+    if (CLUSTER) clusterArrive();
+    else if (nblk > 1) gridArrive(mail, ++epoch, nblk);
+    else __syncthreads();
+    e = firstOf(d);
+    if (CLUSTER) clusterWait();
+    else if (nblk > 1 && !gridWait(mail, epoch, barWords + kExtrapError, nblk)) return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) barWords[3] = (unsigned)(d - 1);
+  if (blockIdx.x == 0 && threadIdx.x == 0) barWords[kExtrapDepth] = (unsigned)(d - 1);
 }
 
 namespace {
@@ -641,37 +792,50 @@ CoopLease::~CoopLease() {
   g_coopFree.notify_all();
 }
 
-// Layers 1 .. nums-1 in one cooperative launch: about one block per 8192
-// faces of the grids, at most kExtrapPerSM per SM, and at most an equal
-// share of the GPU's resident slots for this kernel among the registered
-// users, so that the grids of concurrent scenes always fit on the GPU
-// together.
+// The layers' launch.  Grids of at most kExtrapClusterFaces faces: one cluster
+// of 16 blocks (8 where the device has no 16), whose barrier and values stay
+// within one GPC: a layer of 64^3 takes 3.0 us instead of 4.7; the L2 bandwidth
+// of 16 SMs is what limits it on larger grids.  Those take a cooperative grid: about one
+// block per 4096 faces, at most one per SM, and at most an equal share of the
+// GPU's resident slots for this kernel among the registered users, so that
+// the grids of concurrent scenes always fit on the GPU together.
+// Whole calls in us, cluster / cooperative grid: 64^3 294 / 400, 96^3 (2.7 M
+// faces) 553 / 581, 128^3 (6.3 M) 927 / 806, 256^3 5333 / 2612; hence the line.
+constexpr long long kExtrapClusterFaces = 3000000;
 cudaError_t launchExtrapLayers(const Dim3i rc[3], float* const vals[3], const long long off[3], ExtrapScratch sc,
                                int nums, cudaStream_t s, long long* launches) {
   if (nums <= 1) return cudaSuccess;
+  const long long faces = rc[0].size() + rc[1].size() + rc[2].size();
+  ExtrapGrids g = extrapGrids(rc, vals, off);
+  const uint8_t* mask = sc.mask;
+  const unsigned int* list = sc.list;
+  const unsigned int* offs = sc.offsets;
+  unsigned* bar = extrapBarWords(sc);
+  cudaError_t e;
+  if (faces <= kExtrapClusterFaces) {
+    int size = 0;
+    if ((e = clusterSize((const void*)kExtrapLayers<true>, kExtrapThreads, 0, &size)) != cudaSuccess) return e;
+    if (size > 0) {
+      // small grids need fewer blocks than the cluster could have
+      while (size > 1 && (long long)(size / 2) * kExtrapThreads * 16 >= faces) size /= 2;
+      e = launchCluster(kExtrapLayers<true>, size, kExtrapThreads, 0, s, g, mask, list, offs, nums, bar);
+      if (e == cudaSuccess && launches) ++*launches;
+      return e;
+    }
+  }
   static std::atomic<int> perSM{0};
   if (perSM.load() == 0) {
     int v = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kExtrapLayers, kExtrapThreads, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kExtrapLayers<false>, kExtrapThreads, 0);
     if (e != cudaSuccess) return e;
     perSM.store(std::max(1, v));
   }
   const long long slots = (long long)numSMs() * perSM.load();
   const long long share = std::max(1LL, slots / std::max(1, g_extrapUsers.load()));
-  const long long faces = rc[0].size() + rc[1].size() + rc[2].size();
   const int blocks = (int)std::max(
-      1LL,
-      std::min({(faces + 8191) / 8192, (long long)numSMs() * std::min(perSM.load(), kExtrapPerSM), share}));
-  Dim3i r0 = rc[0], r1 = rc[1], r2 = rc[2];
-  float *v0 = vals[0], *v1 = vals[1], *v2 = vals[2];
-  unsigned o1 = (unsigned)off[1], o2 = (unsigned)off[2];
-  const uint8_t* mask = sc.mask;
-  const unsigned int* list = sc.list;
-  const unsigned int* offs = sc.offsets;
-  unsigned* bar = extrapBarWords(sc);
-  void* args[] = {&r0, &r1, &r2, &v0, &v1, &v2, &o1, &o2, &mask, &list, &offs, &nums, &bar};
-  cudaError_t e =
-      cudaLaunchCooperativeKernel((const void*)kExtrapLayers, dim3(blocks), dim3(kExtrapThreads), args, 0, s);
+      1LL, std::min({(faces + 4095) / 4096, (long long)numSMs(), share, (long long)kExtrapMaxBlocks}));
+  void* args[] = {&g, &mask, &list, &offs, &nums, &bar};
+  e = cudaLaunchCooperativeKernel((const void*)kExtrapLayers<false>, dim3(blocks), dim3(kExtrapThreads), args, 0, s);
   if (e == cudaSuccess && launches) ++*launches;
   return e;
 }
@@ -2147,12 +2311,13 @@ __global__ void kSelftestMbarrier(unsigned long long waitNs, int* out) {
   }
 }
 __global__ void kSelftestGridBarrier(unsigned* words, int* out) {
-  // words: count, generation, error
-  const bool ok = gridBarrier(words, words + 1, words + 2, gridDim.x + 1);
+  // words: error, then three mailboxes (the third block does not exist)
+  gridArrive(words + 1, 1u, gridDim.x + 1);
+  const bool ok = gridWait(words + 1, 1u, words, gridDim.x + 1);
   if (threadIdx.x == 0 && blockIdx.x == 0) out[1] = ok ? 0 : 1;
 }
 cudaError_t launchSelftestWaits(unsigned long long waitNs, unsigned* words, int* out, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(words, 0, 3 * sizeof(unsigned), s);
+  cudaError_t e = cudaMemsetAsync(words, 0, 10 * sizeof(unsigned), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(out, 0xff, 2 * sizeof(int), s);
   if (e != cudaSuccess) return e;
   kSelftestMbarrier<<<1, 32, 0, s>>>(waitNs, out);

@@ -245,18 +245,20 @@ struct ExtrapScratch {
                            // down, up, back, front) that lie in an earlier layer
 };
 constexpr int kMaxLayers = 1000;
-// hist[0 .. kMaxLayers + 1] is the histogram; hist[kMaxLayers + 2 ..] the
-// barrier count, generation and error word of the layer kernel
-constexpr int kExtrapHistWords = kMaxLayers + 2 + 4;
+// hist[0 .. kMaxLayers + 1] is the histogram; hist[kMaxLayers + 2 ..] the words
+// of the layer kernel
+constexpr int kExtrapMaxBlocks = 192;  // blocks of one launch, at most
+constexpr int kExtrapError = 0, kExtrapDepth = 1, kExtrapSlots = 4;  // of the barrier words
+constexpr int kExtrapHistWords = kMaxLayers + 2 + kExtrapSlots + kExtrapMaxBlocks * kExtrapMaxBlocks;
 cudaError_t launchExtrapDistance(const Dim3i rc[3], float* const vals[3], long long off[3], int nums,
                                  ExtrapScratch sc, cudaStream_t s);
 // a layer of at most this many faces is filled by one block (runs of such
 // layers without grid barriers between them)
 constexpr unsigned kExtrapSmallLayer = 4096;
-// Every layer 1 .. nums-1 in one cooperative launch, with a grid barrier
-// between layers.  The barrier waits are bounded.  Afterwards the four words
-// at extrapBarWords() hold: count, generation, error (nonzero: a barrier timed
-// out and the layers are incomplete), deepest layer filled.
+// Every layer 1 .. nums-1 in one launch, with a barrier over its blocks
+// between layers.  The barrier waits are bounded.  Afterwards the words
+// at extrapBarWords() hold kExtrapError (nonzero: a barrier timed out and the
+// layers are incomplete) and kExtrapDepth, the deepest layer filled.
 cudaError_t launchExtrapLayers(const Dim3i rc[3], float* const vals[3], const long long off[3], ExtrapScratch sc,
                                int nums, cudaStream_t s, long long* launches);
 inline unsigned int* extrapBarWords(const ExtrapScratch& sc) { return sc.hist + kMaxLayers + 2; }

@@ -807,13 +807,13 @@ void GridSolver::extrapolate() {
     float* vals[3] = {vel_[ni][0].p, vel_[ni][1].p, vel_[ni][2].p};
     long long off[3] = {0, F_[0], F_[0] + F_[1]};
     ExtrapScratch sc{dist_.p, list_.p, hist_.p, offsets_.p, cursor_.p, mask_.p};
-    launched(launchExtrapDistance(fr_, vals, off, nums, sc, stream_), "extrapolation distance", 17);
+    launched(launchExtrapDistance(fr_, vals, off, nums, sc, stream_), "extrapolation distance", 6);
     CoopLease lease(false);
     check(launchExtrapLayers(fr_, vals, off, sc, nums, stream_, &launches_), "extrapolation layers");
     readBack(extrapHost_, extrapBarWords(sc), sizeof(unsigned int) * 4, stream_);
     check(cudaStreamSynchronize(stream_), "extrapolation sync");
-    if (extrapHost_[2] != 0u) throw CudaError("extrapolation: a grid barrier timed out", HFG_ERR_TIMEOUT);
-    extrapDepth_ = (int)extrapHost_[3];
+    if (extrapHost_[kExtrapError] != 0u) throw CudaError("extrapolation: a grid barrier timed out", HFG_ERR_TIMEOUT);
+    extrapDepth_ = (int)extrapHost_[kExtrapDepth];
   }
   stageEnd(7);
 }

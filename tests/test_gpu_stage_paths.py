@@ -109,6 +109,23 @@ def test_fluid_distance_field(cuda, res, layers):
     assert np.array_equal(host(out), ref)
 
 
+# --- extrapolation: means in a fixed order, so exact --------------------------
+@pytest.mark.parametrize("res", [(1, 1, 1), (31, 2, 3), (33, 17, 1), (40, 129, 3), (257, 9, 5),
+                                 (90, 80, 60), (101, 100, 102)])
+def test_extrapolation_shapes(cuda, res):
+    """Both forms of the layer pass (one cluster up to 3 M faces, a grid above)."""
+    rng = np.random.default_rng(res[1])
+    v = [rng.standard_normal(s).astype(np.float32) for s in oracle.face_shapes(res)]
+    for a in v:
+        a[rng.random(a.shape) < (0.97 if a.size < 10000 else 0.9999)] = UNKNOWN
+        a.flat[0] = 1.0
+    for layers in (2, 7, 1000) if res[0] < 90 else (1000,):
+        vd = [dev(a) for a in v]
+        hfgrid.op_extrapolate_fc(res, vd, layers)
+        for x, y in zip(vd, oracle.extrapolate_fc(res, v, layers)):
+            assert np.array_equal(host(x), y)
+
+
 # --- transfers ------------------------------------------------------------------
 @pytest.mark.parametrize("alg", [hfgrid.LINEAR, hfgrid.QUADRATIC, hfgrid.CUBIC])
 @pytest.mark.parametrize("res", [(1, 1, 1), (2, 3, 1), (8, 5, 6), (13, 4, 7)])
