@@ -659,7 +659,15 @@ HFG_API int hfg_op_project(const int res[3], const float spacing[3], float dt, c
       check(cudaMemcpyAsync(&host, cs.p, sizeof(host), cudaMemcpyDeviceToHost, s), "read state");
       check(cudaStreamSynchronize(s), "sync");
     };
-    if (cgResidentEligible(cg, init.precond, false)) {
+    if (cgClusterEligible(cg, init.precond, false)) {
+      do {
+        check(launchCgCluster(cg, sx, sy, sz, cgc.p, r.p, x.p, p0.p, p1.p, cs.p, init.precond, sched.p, kResidentIters,
+                              s),
+              "cluster cg");
+        readState();
+      } while (!host.done && host.resident == 1);
+    }
+    if (!host.done && cgResidentEligible(cg, init.precond, false)) {
       CoopLease lease(true);
       Scratch<uint8_t> box(lease.held() ? cgResidentBytes(cg) : 0, s);
       if (lease.held()) do {

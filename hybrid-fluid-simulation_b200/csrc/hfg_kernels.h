@@ -192,6 +192,13 @@ size_t cgResidentBytes(const Dim3i& cg);
 cudaError_t launchCgResident(const Dim3i& cg, float sx, float sy, float sz, const CgCode* code, float* r, float* x,
                              float* p, float* zG, void* mailboxes, CgState* st, int precond, const int* sched,
                              int maxIters, cudaStream_t s);
+// The same for small systems as one thread block cluster, which the hardware
+// schedules whole: no lease and no mailboxes.  CgState::resident is 2 where the
+// system is too large for it.
+bool cgClusterEligible(const Dim3i& cg, int precond, bool xDouble);
+cudaError_t launchCgCluster(const Dim3i& cg, float sx, float sy, float sz, const CgCode* code, float* r, float* x,
+                            float* p, float* zG, CgState* st, int precond, const int* sched, int maxIters,
+                            cudaStream_t s);
 // Kernels whose blocks wait on one another must be resident together.  Those
 // that take a share of the GPU (launchExtrapLayers) hold a shared lease from
 // before the launch until the stream has been synchronised after it; one that

@@ -664,6 +664,16 @@ void GridSolver::runCg() {
 // does not fit.
 bool GridSolver::runCgResident(float sx, float sy, float sz, int pc) {
   if (!cgResidentEligible(cg_, pc, xDouble())) return false;
+  if (cgClusterEligible(cg_, pc, xDouble())) {
+    do {
+      launched(launchCgCluster(cg_, sx, sy, sz, cgc_.p, cgr_.p, cgx_.p, cgp_[0].p, cgp_[1].p, cgState_.p, pc, colZ_.p,
+                               kResidentIters, stream_),
+               "cluster cg");
+      readBack(cgHost_, cgState_.p, sizeof(CgState), stream_);
+      check(cudaStreamSynchronize(stream_), "cg sync");
+    } while (!cgHost_->done && cgHost_->resident == 1);
+    if (cgHost_->done) return true;
+  }
   CoopLease lease(true);
   if (!lease.held()) return false;
   cgBox_.alloc(cgResidentBytes(cg_), stream_);
