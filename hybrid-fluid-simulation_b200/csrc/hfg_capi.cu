@@ -7,6 +7,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "hfg_solver.h"
 
@@ -129,6 +130,23 @@ template <class T> struct Scratch {
   }
   ~Scratch() {
     if (p) cudaFreeAsync(p, s);
+  }
+};
+// Several arrays in one allocation, each on 256 bytes.
+struct Arena {
+  std::vector<size_t> at;
+  Scratch<uint8_t> mem;
+  Arena(cudaStream_t s, std::initializer_list<size_t> bytes) : mem(layout(bytes, at), s) {}
+  template <class T> T* get(int i) const { return reinterpret_cast<T*>(mem.p + at[i]); }
+
+ private:
+  static size_t layout(std::initializer_list<size_t> bytes, std::vector<size_t>& at) {
+    size_t n = 0;
+    for (size_t b : bytes) {
+      at.push_back(n);
+      n += (b + 255) & ~(size_t)255;
+    }
+    return n > 0 ? n : 256;
   }
 };
 }  // namespace
@@ -629,75 +647,80 @@ HFG_API int hfg_op_project(const int res[3], const float spacing[3], float dt, c
     const Dim3i cg = cgDims(g.r);
     long long N = g.r.size(), NC = cg.size();
     cudaStream_t s = st(stream);
-    Scratch<Code> code(NC, s);
-    Scratch<CgCode> cgc(NC, s);
-    Scratch<float> r(NC, s), x(NC, s), p0(NC, s), p1(NC, s);
-    Scratch<double> part(cgPartialsNeeded(g.r), s);
-    Scratch<CgState> cs(1, s);
+    const Arena ar(s, {sizeof(Code) * NC, sizeof(CgCode) * NC, sizeof(float) * NC, sizeof(float) * NC,
+                       sizeof(float) * NC, sizeof(float) * NC, sizeof(double) * cgPartialsNeeded(g.r),
+                       sizeof(CgState), sizeof(int) * cgScheduleInts(cg),
+                       cgResidentEligible(cg, precond, false) ? cgResidentBytes(cg) : 0});
+    Code* code = ar.get<Code>(0);
+    CgCode* cgc = ar.get<CgCode>(1);
+    float *r = ar.get<float>(2), *x = ar.get<float>(3), *p0 = ar.get<float>(4), *p1 = ar.get<float>(5);
+    double* part = ar.get<double>(6);
+    CgState* cs = ar.get<CgState>(7);
+    int* sched = ar.get<int>(8);
+    uint8_t* box = ar.get<uint8_t>(9);
     CgMaps maps;
-    check(makeCgMaps(cg, cgc.p, r.p, x.p, false, p0.p, p1.p, &maps), "tensor maps");
+    check(makeCgMaps(cg, cgc, r, x, false, p0, p1, &maps), "tensor maps");
     CgState init{};
     init.maxIter = (int)std::min<long long>(max_iter < 0 ? N : max_iter, 0x7fffffff);
     init.precond = precond == HFG_PRECOND_JACOBI ? 1 : 0;
     init.tolMode = tol_mode;
     init.tol = tol;
-    check(cudaMemcpyAsync(cs.p, &init, sizeof(init), cudaMemcpyHostToDevice, s), "state");
+    check(cudaMemcpyAsync(cs, &init, sizeof(init), cudaMemcpyHostToDevice, s), "state");
     float sx, sy, sz;
     scalesA(spacing, dt, sx, sy, sz);
-    check(launchStencilCode(g.r, cg.x, markers, code.p, s, cgc.p), "code");
+    check(launchStencilCode(g.r, cg.x, markers, code, s, cgc), "code");
     ConstFaceField v{{vx, vy, vz}}, sv{{svx, svy, svz}};
     SolidVelTable none{};
-    check(launchRhsInit(g, v, sv, none, markers, code.p, sx, sy, sz, nullptr, r.p, x.p, false, p0.p, part.p, cs.p,
+    check(launchRhsInit(g, v, sv, none, markers, code, sx, sy, sz, nullptr, r, x, false, p0, part, cs,
                         init.precond, s),
           "rhs");
     // the CG kernels never store at non-fluid cells: both directions start zero
-    check(cudaMemsetAsync(p1.p, 0, sizeof(float) * NC, s), "memset");
-    Scratch<int> sched(cgScheduleInts(cg), s);
-    check(launchCgSchedule(cg, cgc.p, sched.p, init.precond, false, s), "cg schedule");
+    check(cudaMemsetAsync(p1, 0, sizeof(float) * NC, s), "memset");
+    check(launchCgSchedule(cg, cgc, sched, init.precond, false, s), "cg schedule");
     CgState host{};
     auto readState = [&] {
-      check(cudaMemcpyAsync(&host, cs.p, sizeof(host), cudaMemcpyDeviceToHost, s), "read state");
+      check(cudaMemcpyAsync(&host, cs, sizeof(host), cudaMemcpyDeviceToHost, s), "read state");
       check(cudaStreamSynchronize(s), "sync");
     };
     if (cgClusterEligible(cg, init.precond, false)) {
       do {
-        check(launchCgCluster(cg, sx, sy, sz, cgc.p, r.p, x.p, p0.p, p1.p, cs.p, init.precond, sched.p, kResidentIters,
-                              s),
+        check(launchCgCluster(cg, sx, sy, sz, cgc, r, x, p0, p1, cs, init.precond, sched, kResidentIters, s),
               "cluster cg");
         readState();
       } while (!host.done && host.resident == 1);
     }
     if (!host.done && cgResidentEligible(cg, init.precond, false)) {
       CoopLease lease(true);
-      Scratch<uint8_t> box(lease.held() ? cgResidentBytes(cg) : 0, s);
       if (lease.held()) do {
-          check(launchCgResident(cg, sx, sy, sz, cgc.p, r.p, x.p, p0.p, p1.p, box.p, cs.p, init.precond, sched.p,
-                                 kResidentIters, s),
-                "resident cg");
+          const cudaError_t e = launchCgResident(cg, sx, sy, sz, cgc, r, x, p0, p1, box, cs, init.precond,
+                                                 sched, kResidentIters, s);
+          if (cgResidentRefused(e)) break;
+          check(e, "resident cg");
           readState();
         } while (!host.done && host.resident == 1);
     }
-    float* pb[2] = {p0.p, p1.p};
+    float* pb[2] = {p0, p1};
     int it = 0;
     while (!host.done) {
       for (int k = 0; k < 16; ++k, ++it) {
         const int po = it & 1, pn = (it + 1) & 1;
-        check(launchCgDirection(cg, sx, sy, sz, maps.rH, maps.pH[po], maps.codeH, cgc.p, r.p, pb[po], pb[pn], part.p,
-                                cs.p, init.precond, s, sched.p),
+        check(launchCgDirection(cg, sx, sy, sz, maps.rH, maps.pH[po], maps.codeH, cgc, r, pb[po], pb[pn], part,
+                                cs, init.precond, s, sched),
               "cg");
-        check(launchCgUpdate(cg, sx, sy, sz, maps.pH[pn], maps.rI, maps.xI, maps.codeI, pb[pn], x.p, false, r.p, part.p,
-                             cs.p, init.precond, s, sched.p),
+        check(launchCgUpdate(cg, sx, sy, sz, maps.pH[pn], maps.rI, maps.xI, maps.codeI, pb[pn], x, false, r, part,
+                             cs, init.precond, s, sched),
               "cg");
       }
       readState();
     }
+    if (host.error == 4) return fail(HFG_ERR_STATE, "pressure CG: a work item of the schedule is invalid");
     if (host.error) return fail(HFG_ERR_TIMEOUT, "pressure CG: a wait did not complete in time");
     FaceField vv{{vx, vy, vz}};
     check(launchGradient(g, dt / (1.0f * spacing[0]), dt / (1.0f * spacing[1]), dt / (1.0f * spacing[2]), markers,
-                         x.p, false, vv, sv, none, s),
+                         x, false, vv, sv, none, s),
           "gradient");
     if (pOut)
-      check(cudaMemcpy2DAsync(pOut, (size_t)g.r.x * 4, x.p, (size_t)cg.x * 4, (size_t)g.r.x * 4,
+      check(cudaMemcpy2DAsync(pOut, (size_t)g.r.x * 4, x, (size_t)cg.x * 4, (size_t)g.r.x * 4,
                               (size_t)g.r.y * g.r.z, cudaMemcpyDeviceToDevice, s),
             "copy");
     check(cudaStreamSynchronize(s), "sync");
@@ -720,10 +743,10 @@ int extrapolateGrids(int ngrids, const Dim3i* rc, float* const* vals, int layers
   float* v3[3] = {vals[0], vals[0], vals[0]};
   for (int a = 0; a < ngrids; ++a) { off[a] = total; total += rc[a].size(); r3[a] = rc[a]; v3[a] = vals[a]; }
   for (int a = ngrids; a < 3; ++a) { off[a] = total; r3[a] = Dim3i{1, 1, 0}; }
-  Scratch<uint16_t> dist(total, s);
-  Scratch<unsigned int> list(total, s), hist(kExtrapHistWords, s), offs(kMaxLayers + 2, s), cur(kMaxLayers + 2, s);
-  Scratch<uint8_t> mask(total, s);
-  ExtrapScratch sc{dist.p, list.p, hist.p, offs.p, cur.p, mask.p};
+  const Arena ar(s, {sizeof(uint16_t) * total, sizeof(unsigned) * total, sizeof(unsigned) * kExtrapHistWords,
+                     sizeof(unsigned) * (kMaxLayers + 2), sizeof(unsigned) * (kMaxLayers + 2), (size_t)total});
+  ExtrapScratch sc{ar.get<uint16_t>(0), ar.get<unsigned>(1), ar.get<unsigned>(2),
+                   ar.get<unsigned>(3), ar.get<unsigned>(4), ar.get<uint8_t>(5)};
   if (layers > kMaxLayers) layers = kMaxLayers;
   if (layers <= 1) return HFG_OK;
   // grids with zero size contribute nothing
@@ -861,21 +884,23 @@ HFG_API int hfg_op_advect_particles(const int res[3], const float origin[3], con
     Geom g = toGeom(res, origin, spacing);
     cudaStream_t s = st(stream);
     const int slots = 4096;
-    Scratch<SubstepState> ss(slots + 1, s);
-    Scratch<float> v0(3 * (n > 0 ? n : 1), s);
-    check(cudaMemsetAsync(ss.p, 0, sizeof(SubstepState) * (slots + 1), s), "memset");
-    Scratch<float4> q0(faceQuadCount(g.r, 0), s), q1(faceQuadCount(g.r, 1), s), q2(faceQuadCount(g.r, 2), s);
-    float4* quads[3] = {q0.p, q1.p, q2.p};
+    const Arena ar(s, {sizeof(SubstepState) * (slots + 1), sizeof(float) * 3 * (n > 0 ? n : 1),
+                       sizeof(float4) * faceQuadCount(g.r, 0), sizeof(float4) * faceQuadCount(g.r, 1),
+                       sizeof(float4) * faceQuadCount(g.r, 2)});
+    SubstepState* ss = ar.get<SubstepState>(0);
+    float* v0 = ar.get<float>(1);
+    check(cudaMemsetAsync(ss, 0, sizeof(SubstepState) * (slots + 1), s), "memset");
+    float4* quads[3] = {ar.get<float4>(2), ar.get<float4>(3), ar.get<float4>(4)};
     check(launchFaceQuads(g.r, ConstFaceField{{vx, vy, vz}}, quads, s), "face corner tables");
-    FaceQuads v = makeFaceQuads(g, q0.p, q1.p, q2.p);
-    check(launchSubstepBegin(g, v, pos, v0.p, n, ss.p, s), "substep");
+    FaceQuads v = makeFaceQuads(g, quads[0], quads[1], quads[2]);
+    check(launchSubstepBegin(g, v, pos, v0, n, ss, s), "substep");
     long long nclamp = clamp_mode == 1 ? std::min<long long>(n, g.r.size()) : n;
     SubstepState host{};
     int slot = 0;
     for (;;) {
       for (int k = 0; k < 4 && slot < slots; ++k, ++slot)
-        check(launchSubstep(g, v, pos, v0.p, n, accuracy, dt, cfl, nclamp, ss.p, slot, s), "substep");
-      check(cudaMemcpyAsync(&host, ss.p + slot, sizeof(host), cudaMemcpyDeviceToHost, s), "read");
+        check(launchSubstep(g, v, pos, v0, n, accuracy, dt, cfl, nclamp, ss, slot, s), "substep");
+      check(cudaMemcpyAsync(&host, ss + slot, sizeof(host), cudaMemcpyDeviceToHost, s), "read");
       check(cudaStreamSynchronize(s), "sync");
       if (host.finished) break;
       if (slot >= slots) return fail(HFG_ERR_STATE, "CFL substep limit reached");

@@ -289,7 +289,7 @@ struct FaceSampler {
 // edge ones already; a coordinate that is not finite makes every weight, and
 // so every sample, NaN.
 struct LerpGrid {
-  float inv[3], o[3], hi[3];
+  float inv[3], h[3], o[3], hi[3];
   int n[3];
 };
 inline LerpGrid makeLerpGrid(const Geom& g) {
@@ -298,6 +298,7 @@ inline LerpGrid makeLerpGrid(const Geom& g) {
   const int n[3] = {g.r.x, g.r.y, g.r.z};
   for (int k = 0; k < 3; ++k) {
     q.inv[k] = 1.0f / h[k];
+    q.h[k] = h[k];
     q.o[k] = o[k];
     q.hi[k] = std::nextafter((float)n[k] + 0.5f, 0.0f);
     q.n[k] = n[k];
@@ -311,7 +312,9 @@ struct LerpSampler {
     const float p[3] = {px, py, pz};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float u = (p[k] - q.o[k]) * q.inv[k];
+      // the quotient by h: the product with the reciprocal, and its remainder
+      // once more, so that the reciprocal's rounding does not scale the error
+      const float d = p[k] - q.o[k], u0 = d * q.inv[k], u = fmaf(fmaf(-u0, q.h[k], d), q.inv[k], u0);
       const float t = fminf(fmaxf(u, -0.5f), q.hi[k]);
       const float f = floorf(t);
       const float w = (t - f) + (u - u);

@@ -768,26 +768,32 @@ void extrapUsers(int delta) { g_extrapUsers.fetch_add(delta); }
 namespace {
 std::mutex g_coopMu;
 std::condition_variable g_coopFree;
-int g_coopShared = 0;
-bool g_coopExclusive = false;
+struct Coop {
+  int shared = 0;
+  bool exclusive = false;
+};
+std::map<int, Coop> g_coop;  // by device
 }  // namespace
 
-CoopLease::CoopLease(bool exclusive) : exclusive_(exclusive), held_(true) {
+CoopLease::CoopLease(bool exclusive) : exclusive_(exclusive), held_(true), dev_(0) {
+  cudaGetDevice(&dev_);
   std::unique_lock<std::mutex> lk(g_coopMu);
+  Coop& c = g_coop[dev_];
   if (exclusive) {
-    held_ = !g_coopExclusive && g_coopShared == 0;
-    if (held_) g_coopExclusive = true;
+    held_ = !c.exclusive && c.shared == 0;
+    if (held_) c.exclusive = true;
   } else {
-    g_coopFree.wait(lk, [] { return !g_coopExclusive; });
-    ++g_coopShared;
+    g_coopFree.wait(lk, [&] { return !c.exclusive; });
+    ++c.shared;
   }
 }
 CoopLease::~CoopLease() {
   if (!held_) return;
   {
     std::lock_guard<std::mutex> lk(g_coopMu);
-    if (exclusive_) g_coopExclusive = false;
-    else --g_coopShared;
+    Coop& c = g_coop[dev_];
+    if (exclusive_) c.exclusive = false;
+    else --c.shared;
   }
   g_coopFree.notify_all();
 }

@@ -192,6 +192,13 @@ size_t cgResidentBytes(const Dim3i& cg);
 cudaError_t launchCgResident(const Dim3i& cg, float sx, float sy, float sz, const CgCode* code, float* r, float* x,
                              float* p, float* zG, void* mailboxes, CgState* st, int precond, const int* sched,
                              int maxIters, cudaStream_t s);
+// whether a launch failed because the device, as this context sees it, does not
+// hold the whole grid at once (the error is cleared: the kernel pair solves)
+inline bool cgResidentRefused(cudaError_t e) {
+  if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return false;
+  cudaGetLastError();
+  return true;
+}
 // The same for small systems as one thread block cluster, which the hardware
 // schedules whole: no lease and no mailboxes.  CgState::resident is 2 where the
 // system is too large for it.
@@ -202,7 +209,8 @@ cudaError_t launchCgCluster(const Dim3i& cg, float sx, float sy, float sz, const
 // Kernels whose blocks wait on one another must be resident together.  Those
 // that take a share of the GPU (launchExtrapLayers) hold a shared lease from
 // before the launch until the stream has been synchronised after it; one that
-// takes every SM holds the exclusive lease, which is only ever tried for.
+// takes every SM holds the exclusive lease, which is only ever tried for.  The
+// leases are the current device's.
 class CoopLease {
  public:
   explicit CoopLease(bool exclusive);  // shared: waits for an exclusive holder to finish
@@ -213,6 +221,7 @@ class CoopLease {
 
  private:
   bool exclusive_, held_;
+  int dev_;
 };
 // Divergence residual of the projected velocity over the fluid cells:
 // *sumOut = sum b^2 (FP64), ticketAndMax[1] = bits of max |b|.  `scratch`

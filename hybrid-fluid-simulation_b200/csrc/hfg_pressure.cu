@@ -6,7 +6,8 @@
 // host reads per iteration (CuMatrixFreePCG.cpp:22-65).  Here A is rebuilt in
 // registers from a 16-bit stencil code per cell, every CG iteration is two
 // kernels with FP64 block reductions finished by the last block (no host
-// round trip), and the stencil kernels are 2.5-D: a 32x8 thread tile marches
+// round trip), or, where the fluid fits the GPU's shared memory, a whole solve
+// is one launch (the resident CG below), and the stencil kernels are 2.5-D: a 32x8 thread tile marches
 // along z keeping the below / current / above planes in registers, so the z
 // neighbours cost no extra loads and no division is needed for indexing.
 #include <algorithm>
@@ -1663,11 +1664,19 @@ int residentGrid(const Dim3i& cg) {
 }  // namespace
 // Shared memory of a cluster block: RG kResKL planes of up to 8 segments.
 constexpr int kResClusterBytes = (RG * kResKL + 2 * 8) * RPL * 4 + RG * kResKL * CTX * CTR;
+namespace {
+const void* clusterKernel(int precond) {
+  return precond == 1 ? (const void*)kCgResident<1, true> : (const void*)kCgResident<0, true>;
+}
+}  // namespace
 bool cgClusterEligible(const Dim3i& cg, int precond, bool xDouble) {
   // the fluid is seldom more than a quarter of the grid's planes; a system
   // that turns out too large costs one launch and one host read
-  return cgResidentEligible(cg, precond, xDouble) &&
-         (long long)cgColumns(cg) * cg.z <= 4LL * kResCluster * RG * kResKL;
+  if (!cgResidentEligible(cg, precond, xDouble) ||
+      (long long)cgColumns(cg) * cg.z > 4LL * kResCluster * RG * kResKL)
+    return false;
+  int size = 0;
+  return clusterSize(clusterKernel(precond), RTH, kResClusterBytes, &size) == cudaSuccess && size > 0;
 }
 cudaError_t launchCgCluster(const Dim3i& cg, float sx, float sy, float sz, const CgCode* code, float* r, float* x,
                             float* p, float* zG, CgState* st, int precond, const int* sched, int maxIters,
@@ -1676,7 +1685,6 @@ cudaError_t launchCgCluster(const Dim3i& cg, float sx, float sy, float sz, const
   int size = 0;
   cudaError_t e = clusterSize((const void*)k, RTH, kResClusterBytes, &size);
   if (e != cudaSuccess) return e;
-  if (size == 0) return cudaErrorNotSupported;
   const long long planes = (long long)cgColumns(cg) * cg.z;
   while (size > 1 && (long long)(size / 2) * kResMinPlanes >= planes) size /= 2;
   ResArgs A{cg, sx, sy, sz, code, r, x, p, zG, nullptr, st, maxIters};

@@ -678,9 +678,10 @@ bool GridSolver::runCgResident(float sx, float sy, float sz, int pc) {
   if (!lease.held()) return false;
   cgBox_.alloc(cgResidentBytes(cg_), stream_);
   do {
-    launched(launchCgResident(cg_, sx, sy, sz, cgc_.p, cgr_.p, cgx_.p, cgp_[0].p, cgp_[1].p, cgBox_.p, cgState_.p,
-                              pc, colZ_.p, kResidentIters, stream_),
-             "resident cg");
+    const cudaError_t e = launchCgResident(cg_, sx, sy, sz, cgc_.p, cgr_.p, cgx_.p, cgp_[0].p, cgp_[1].p, cgBox_.p,
+                                           cgState_.p, pc, colZ_.p, kResidentIters, stream_);
+    if (cgResidentRefused(e)) return false;
+    launched(e, "resident cg");
     readBack(cgHost_, cgState_.p, sizeof(CgState), stream_);
     check(cudaStreamSynchronize(stream_), "cg sync");
   } while (!cgHost_->done && cgHost_->resident == 1);
