@@ -176,6 +176,7 @@ class GridSolver {
   void p2gFace(const float* vel, float* const out[3], float* const copy[3], const float add[3], bool doAdd,
                const float add2[3], bool doAdd2);
   void p2gScalars(float* const out[4]);
+  void upload(DArray<float>& b0, DArray<float>& b1, const float* host, long long n, const char* what);
   void computePressure();
   void runCg();
   bool runCgResident(float sx, float sy, float sz, int pc);
