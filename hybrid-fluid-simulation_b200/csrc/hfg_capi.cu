@@ -707,7 +707,7 @@ HFG_API int hfg_op_project(const int res[3], const float spacing[3], float dt, c
         check(launchCgDirection(cg, sx, sy, sz, maps.rH, maps.pH[po], maps.codeH, cgc, r, pb[po], pb[pn], part,
                                 cs, init.precond, s, sched),
               "cg");
-        check(launchCgUpdate(cg, sx, sy, sz, maps.pH[pn], maps.rI, maps.xI, maps.codeI, pb[pn], x, false, r, part,
+        check(launchCgUpdate(cg, sx, sy, sz, maps.pH[pn], maps.rI, maps.xI, maps.codeI, cgc, pb[pn], x, false, r, part,
                              cs, init.precond, s, sched),
               "cg");
       }

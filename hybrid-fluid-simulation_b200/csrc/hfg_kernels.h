@@ -152,7 +152,7 @@ cudaError_t launchCgDirection(const Dim3i& cg, float sx, float sy, float sz, con
                               const float* pOld, float* pNew, double* partials, CgState* st, int precond,
                               cudaStream_t s, const int* colZ = nullptr, bool xDouble = false);
 cudaError_t launchCgUpdate(const Dim3i& cg, float sx, float sy, float sz, const CUtensorMap& mP, const CUtensorMap& mR,
-                           const CUtensorMap& mX, const CUtensorMap& mCode, const float* p, void* x, bool xDouble,
+                           const CUtensorMap& mX, const CUtensorMap& mCode, const CgCode* code, const float* p, void* x, bool xDouble,
                            float* r, double* partials, CgState* st, int precond, cudaStream_t s,
                            const int* colZ = nullptr);
 // Measured launch shapes of the CG kernels (family 0 direction, 1 update):

@@ -913,6 +913,111 @@ __global__ void __launch_bounds__(CTX* CTY, 4)
   }
 }
 
+// The two kernels on small grids, between the launches of a V-cycle (z from
+// memory): a cell to a thread at a time, every load of a cell in flight at
+// once.  There is nothing to stream on such a grid, and the ring's set-up and
+// fill, the plane barriers and a reduction over many blocks were most of the
+// time: with a V-cycle's launches around them, the
+// CG stage of a 64^3 step 1.43 -> 1.36 ms.  The operations and their order are the marching kernels';
+// neighbours that are solid or outside hold zero and are not loaded, which the
+// cell's code tells without coordinates.
+constexpr long long kCgSmallGrid = 1 << 19;          // cells of a small grid, at most
+constexpr int kSmallThreads = 256, kSmallCells = 4;  // cells of a thread
+struct CgNb {
+  float l, r, d, u, b, f;
+};
+template <class G>
+__device__ __forceinline__ CgNb cgNeighbours(CgCode k, unsigned c, unsigned nx, unsigned plane, G get) {
+  CgNb n;
+  n.l = k & 2 ? get(c - 1) : 0.f;
+  n.r = k & 4 ? get(c + 1) : 0.f;
+  n.d = k & 8 ? get(c - nx) : 0.f;
+  n.u = k & 16 ? get(c + nx) : 0.f;
+  n.b = k & 32 ? get(c - plane) : 0.f;
+  n.f = k & 64 ? get(c + plane) : 0.f;
+  return n;
+}
+__global__ void __launch_bounds__(kSmallThreads)
+    kCgDirectionSmall(Dim3i P, float sx, float sy, float sz, const CgCode* __restrict__ code,
+                      const float* __restrict__ z, const float* __restrict__ pOld, float* __restrict__ pNew,
+                      double* partials, CgState* st) {
+  const unsigned nx = (unsigned)P.x, plane = nx * (unsigned)P.y, n = plane * (unsigned)P.z;
+  const unsigned c0 = blockIdx.x * (kSmallThreads * kSmallCells) + threadIdx.x;
+  CgCode k[kSmallCells];  // the codes do not change within a solve
+#pragma unroll
+  for (int j = 0; j < kSmallCells; ++j) {
+    const unsigned c = c0 + j * kSmallThreads;
+    k[j] = c < n ? __ldg(code + c) : (CgCode)0;
+  }
+  waitPrevGrid();
+  if (st->done) return;
+  allowNextGrid();
+  const float beta = st->beta;
+  auto pAt = [&](unsigned i) { return fmaf(beta, __ldg(pOld + i), __ldg(z + i)); };
+  double acc = 0.0, dummy = 0.0;
+#pragma unroll
+  for (int j = 0; j < kSmallCells; ++j) {
+    if (!(k[j] & 1)) continue;
+    const unsigned c = c0 + j * kSmallThreads;
+    const float pc = pAt(c);
+    const CgNb v = cgNeighbours(k[j], c, nx, plane, pAt);
+    const float q = rowSum(diagOf((Code)k[j], sx, sy, sz), sx, sy, sz, pc, v.l, v.r, v.d, v.u, v.b, v.f);
+    pNew[c] = pc;
+    acc = fma((double)pc, (double)q, acc);
+  }
+  if (gridSum2(acc, dummy, partials, &st->ticket) && flatTid() == 0) {
+    st->pAp = acc;
+    st->alpha = (float)(st->rz / acc);
+    st->ticket = 0;
+  }
+}
+template <class TX>
+__global__ void __launch_bounds__(kSmallThreads)
+    kCgUpdateSmall(Dim3i P, float sx, float sy, float sz, const CgCode* __restrict__ code, const float* __restrict__ p,
+                   TX* __restrict__ x, float* __restrict__ r, double* partials, CgState* st) {
+  const unsigned nx = (unsigned)P.x, plane = nx * (unsigned)P.y, n = plane * (unsigned)P.z;
+  const unsigned c0 = blockIdx.x * (kSmallThreads * kSmallCells) + threadIdx.x;
+  CgCode k[kSmallCells];
+#pragma unroll
+  for (int j = 0; j < kSmallCells; ++j) {
+    const unsigned c = c0 + j * kSmallThreads;
+    k[j] = c < n ? __ldg(code + c) : (CgCode)0;
+  }
+  waitPrevGrid();
+  if (st->done) return;
+  allowNextGrid();
+  const float alpha = st->alpha;
+  const bool skip = fabsf(alpha) < FLT_EPSILON;
+  double rr = 0.0, dummy = 0.0;
+#pragma unroll
+  for (int j = 0; j < kSmallCells; ++j) {
+    if (!(k[j] & 1)) continue;
+    const unsigned c = c0 + j * kSmallThreads;
+    float rv = r[c];
+    if (!skip) {
+      const float pc = __ldg(p + c);
+      const CgNb v = cgNeighbours(k[j], c, nx, plane, [&](unsigned i) { return __ldg(p + i); });
+      const float q = rowSum(diagOf((Code)k[j], sx, sy, sz), sx, sy, sz, pc, v.l, v.r, v.d, v.u, v.b, v.f);
+      if (sizeof(TX) == 8)
+        x[c] = (TX)__dadd_rn((double)x[c], __dmul_rn((double)alpha, (double)pc));
+      else
+        x[c] = (TX)fmaf(alpha, pc, (float)x[c]);
+      rv = fmaf(-alpha, q, rv);
+      r[c] = rv;
+    }
+    rr = fma((double)rv, (double)rv, rr);
+  }
+  if (gridSum2(rr, dummy, partials, &st->ticket) && flatTid() == 0) {
+    st->rr = rr;
+    st->iter += 1;
+    st->done = st->error || cgStop(st, rr) || st->iter >= st->maxIter;
+    st->ticket = 0;
+  }
+}
+int smallBlocks(const Dim3i& cg) {
+  return (int)((cg.size() + kSmallThreads * kSmallCells - 1) / (kSmallThreads * kSmallCells));
+}
+
 // ---------------------------------------------------------------------------
 // The resident CG: whole solves in one cooperative launch, for systems whose
 // fluid fits the shared memory of the GPU.
@@ -1761,6 +1866,9 @@ cudaError_t launchCgDirection(const Dim3i& cg, float sx, float sy, float sz, con
       break;
     }
     case 2: {
+      if (cg.size() <= kCgSmallGrid)
+        return launchPdl(kCgDirectionSmall, dim3(smallBlocks(cg)), dim3(kSmallThreads), s, cg, sx, sy, sz, code, zr, pOld,
+                         pNew, partials, st);
       CgLaunch L = cgLaunch(cg, kCgDirection<2>, 0, colZ, 2, xDouble);
       cudaError_t e = launchPdl(kCgDirection<2>, L.grid, L.block, s, mZ, mPo, mCode, cg, sx, sy, sz, code, zr, pOld,
                                 pNew, partials, st, L.zPer, colZ);
@@ -1778,8 +1886,13 @@ cudaError_t launchCgDirection(const Dim3i& cg, float sx, float sy, float sz, con
 }
 
 cudaError_t launchCgUpdate(const Dim3i& cg, float sx, float sy, float sz, const CUtensorMap& mP, const CUtensorMap& mR,
-                           const CUtensorMap& mX, const CUtensorMap& mCode, const float* p, void* x, bool xDouble,
+                           const CUtensorMap& mX, const CUtensorMap& mCode, const CgCode* code, const float* p, void* x, bool xDouble,
                            float* r, double* partials, CgState* st, int precond, cudaStream_t s, const int* colZ) {
+  if (precond == 2 && cg.size() <= kCgSmallGrid)
+    return xDouble ? launchPdl(kCgUpdateSmall<double>, dim3(smallBlocks(cg)), dim3(kSmallThreads), s, cg, sx, sy, sz,
+                               code, p, (double*)x, r, partials, st)
+                   : launchPdl(kCgUpdateSmall<float>, dim3(smallBlocks(cg)), dim3(kSmallThreads), s, cg, sx, sy, sz,
+                               code, p, (float*)x, r, partials, st);
 #define HFG_CG_UPDATE(PCV, TXV)                                                                                   \
   {                                                                                                               \
     CgLaunch L = cgLaunch(cg, kCgUpdate<PCV, TXV>, 1, colZ, PCV, xDouble);                                                             \

@@ -612,7 +612,7 @@ void GridSolver::cgIteration(int it, float sx, float sy, float sz, int pc) {
   launched(launchCgDirection(cg_, sx, sy, sz, maps_.rH, maps_.pH[po], maps_.codeH, cgc_.p, cgr_.p, cgp_[po].p,
                              cgp_[pn].p, partials_.p, cgState_.p, pc, stream_, colZ_.p, xDouble()),
            "cg direction");
-  launched(launchCgUpdate(cg_, sx, sy, sz, maps_.pH[pn], maps_.rI, maps_.xI, maps_.codeI, cgp_[pn].p, xPtr(), xDouble(),
+  launched(launchCgUpdate(cg_, sx, sy, sz, maps_.pH[pn], maps_.rI, maps_.xI, maps_.codeI, cgc_.p, cgp_[pn].p, xPtr(), xDouble(),
                           cgr_.p,
                           partials_.p, cgState_.p, pc, stream_, colZ_.p),
            "cg update");
@@ -907,7 +907,7 @@ void GridSolver::autotuneCg(float sx, float sy, float sz, int pc) {
                                    cgp_[po].p, cgp_[pn].p, partials_.p, cgState_.p, pc, stream_, colZ_.p, xDouble()),
                  "cg direction");
         check(cudaEventRecord(e[3 * it + 1], stream_), "event");
-        launched(launchCgUpdate(cg_, sx, sy, sz, maps_.pH[pn], maps_.rI, maps_.xI, maps_.codeI, cgp_[pn].p, xPtr(),
+        launched(launchCgUpdate(cg_, sx, sy, sz, maps_.pH[pn], maps_.rI, maps_.xI, maps_.codeI, cgc_.p, cgp_[pn].p, xPtr(),
                                 xDouble(), cgr_.p, partials_.p, cgState_.p, pc, stream_, colZ_.p),
                  "cg update");
         check(cudaEventRecord(e[3 * it + 2], stream_), "event");
