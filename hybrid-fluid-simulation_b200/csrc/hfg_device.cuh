@@ -540,13 +540,33 @@ __device__ inline void taps(const Geom& g, float px, float py, float pz, Taps& t
 
 template <int ALG> struct TapsN { static constexpr int n = (ALG == LINEAR) ? 2 : 4; static constexpr int shift = (ALG == LINEAR) ? 0 : -1; };
 
+// Linear indices of a stencil's taps, clamped to the grid once per axis (every
+// grid holds fewer than 2^32 entries), where clamping and multiplying out each
+// of 64 in 64 bits took issue slots that the 192 gathers of a particle need.
+// G2P of 3.6 M particles on 130x110x137: quadratic 439 -> 323 us, cubic 421 ->
+// 319; of 1.4 M on 97x77x104: 176 -> 133 and 168 -> 131.
+template <int ALG> struct TapRows {
+  static constexpr int n = TapsN<ALG>::n, s = TapsN<ALG>::shift;
+  unsigned xi[n], yi[n], zi[n], nx, ny;
+  __device__ __forceinline__ TapRows(const Geom& g, const Taps& t) : nx((unsigned)g.r.x), ny((unsigned)g.r.y) {
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+      xi[k] = (unsigned)clampi(t.base[0] + k + s, g.r.x);
+      yi[k] = (unsigned)clampi(t.base[1] + k + s, g.r.y);
+      zi[k] = (unsigned)clampi(t.base[2] + k + s, g.r.z);
+    }
+  }
+  __device__ __forceinline__ unsigned operator()(int x, int y, int z) const { return (zi[z] * ny + yi[y]) * nx + xi[x]; }
+};
+
 // G2P of one component (accumulateCCSField2Particles, EulerParticlesTool.cu:198-288)
 template <int ALG>
 __device__ inline float g2p(const float* __restrict__ f, const Geom& g, float px, float py, float pz) {
   if (ALG == G2PNEAREST) return __ldg(f + binCell(g, px, py, pz));
   Taps t;
   taps<ALG>(g, px, py, pz, t);
-  constexpr int n = TapsN<ALG>::n, s = TapsN<ALG>::shift;
+  constexpr int n = TapsN<ALG>::n;
+  TapRows<ALG> at(g, t);
   float acc = 0.f;
 #pragma unroll
   for (int z = 0; z < n; ++z)
@@ -555,7 +575,7 @@ __device__ inline float g2p(const float* __restrict__ f, const Geom& g, float px
 #pragma unroll
       for (int x = 0; x < n; ++x) {
         float w = t.w[0][x] * t.w[1][y] * t.w[2][z];
-        acc += w * __ldg(f + linc(t.base[0] + x + s, t.base[1] + y + s, t.base[2] + z + s, g.r));
+        acc += w * __ldg(f + at(x, y, z));
       }
   return acc;
 }

@@ -1340,7 +1340,8 @@ __global__ void kParticleVelUpdate(Geom g, int mode, ConstFaceField vin, ConstFa
           // G2P of the face-wise difference vin - prev
           Taps t;
           taps<ALG == G2PNEAREST ? LINEAR : ALG>(fg, px, py, pz, t);
-          constexpr int n = TapsN<ALG>::n, sft = TapsN<ALG>::shift;
+          constexpr int A = ALG == G2PNEAREST ? LINEAR : ALG, n = TapsN<A>::n;
+          const TapRows<A> at(fg, t);
           dv = 0.f;
           if (ALG == G2PNEAREST) {
             long long i = binCell(fg, px, py, pz);
@@ -1353,7 +1354,7 @@ __global__ void kParticleVelUpdate(Geom g, int mode, ConstFaceField vin, ConstFa
 #pragma unroll
                 for (int x = 0; x < n; ++x) {
                   float w = t.w[0][x] * t.w[1][y] * t.w[2][z];
-                  long long i = linc(t.base[0] + x + sft, t.base[1] + y + sft, t.base[2] + z + sft, fg.r);
+                  const unsigned i = at(x, y, z);
                   dv += w * __fsub_rn(__ldg(vin.c[a] + i), __ldg(prev.c[a] + i));
                 }
           }
