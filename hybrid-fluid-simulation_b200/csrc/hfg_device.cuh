@@ -163,12 +163,12 @@ struct FaceQuads {
   // Sampling constants of the grid, formed once on the host (makeFaceQuads)
   // so that a kernel reads them as launch parameters: the coordinate of a
   // point on axis k is p * inv + offF on the face grid of that axis and
-  // p * inv + offC (offF - 1/2) on the cell-centred one; jF and jC (n and
-  // n - 1 for n cells) are the largest floor index there, and hi, the float
-  // below n + 1/2, bounds the face coordinate (QuadSampler); lx, ly and pl are
-  // the row length, the rows per layer and the layer size of component a's
-  // table.
-  float inv[3], offF[3], offC[3], hi[3];
+  // p * inv + offC (offF - 1/2) on the cell-centred one; hiF and hiC, the
+  // float below n + 1 and n for n cells, bound the coordinate on those two
+  // grids, and jF and jC (n and n - 1) are the largest floor index there;
+  // lx, ly and pl are the row length, the rows per layer and the layer size
+  // of component a's table.
+  float inv[3], offF[3], offC[3], hiF[3], hiC[3];
   int jF[3], jC[3];
   unsigned lx[3], ly[3], pl[3];
 };
@@ -184,7 +184,8 @@ inline FaceQuads makeFaceQuads(const Geom& g, const float4* q0, const float4* q1
     q.offC[k] = q.offF[k] - 0.5f;
     q.jF[k] = n[k];
     q.jC[k] = n[k] - 1;
-    q.hi[k] = std::nextafter((float)n[k] + 0.5f, 0.0f);
+    q.hiF[k] = std::nextafter((float)(n[k] + 1), 0.0f);
+    q.hiC[k] = std::nextafter((float)n[k], 0.0f);
   }
   for (int a = 0; a < 3; ++a) {
     q.lx[a] = (unsigned)(n[0] + (a == 0) + 1);
@@ -350,18 +351,23 @@ struct LerpSampler {
     return fmaf(wz, d1 - d0, d0);
   }
 };
-// The trilinear sample of the substeps, from the corner tables alone.  The
-// cell-centred coordinate of an axis is its face coordinate less 1/2, so one
-// floor per axis gives both base entries and weights: with w the face weight,
-// (j, w - 1/2) from the middle of a cell on, (j - 1, w + 1/2) before it (both
-// exact but for the last bit of the second).  The floor and its conversion run
-// on the quarter-rate pipe, which took 36 of them per RK3
-// particle-substep with one for each grid and takes 18 now.  A 256^3 step
-// of 23 substeps of 31.4 M particles: 12.6 -> 11.5 ms; 160^3, 7.6 M: 132 ->
-// 124 us a launch.  (Resampling v0 instead of streaming it, 24 of the 48 bytes
-// a particle, cost 0.9 ms a step; no entry cache and 40 warps an SM cost 4.)
-// The coordinate is clamped first to [-1/2, n + 1/2): the bounds of both grids'
-// tables.  A coordinate outside selects the same edge corners as an integer
+// The trilinear sample of the substeps, from the corner tables alone.  Every
+// axis has two coordinates, one on the face grid and one on the cell-centred
+// grid, each one FMA and clamped to its table's bounds; one floor serves both:
+// the cell-centred coordinate is the face coordinate less 1/2, so its floor is
+// the face floor or one less, which a comparison tells.  The floor and its
+// conversion run on the quarter-rate pipe, 36 of them per RK3
+// particle-substep with one for each grid, 18 so.  The weights are those that
+// a floor per coordinate gives, to the bit (up to 2^22 cells from the origin,
+// where 1/2 is still exact): the trajectories of a flow part from a last bit
+// on, so a weight off by one would be another flow.
+// The substeps of a 256^3 step, 31.4 M particles, in ms: 12.5 with a floor per
+// coordinate and four waves of blocks, 11.0 so with one wave (kSubstep); with
+// the cell-centred weight taken from the face weight, whose last bit then
+// differs at one coordinate in 5000, 11.4 at four.  (Resampling v0 instead of
+// streaming it, 24 of the 48 bytes a particle, cost 0.9 ms a step; no entry
+// cache and 40 warps an SM cost 4.)
+// A coordinate outside its bounds selects the same edge corners as an integer
 // clamp would, which hold equal values (the x differences and the y and z
 // corner pairs there are exact zeros), so every finite point samples the same
 // value; a NaN point samples the edge instead of returning NaN.
@@ -372,14 +378,14 @@ struct QuadSampler {
     const float p[3] = {px, py, pz};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float t = fminf(fmaxf(fmaf(p[k], q.inv[k], q.offF[k]), -0.5f), q.hi[k]);
+      const float t = fminf(fmaxf(fmaf(p[k], q.inv[k], q.offF[k]), -1.0f), q.hiF[k]);
+      const float c = fminf(fmaxf(fmaf(p[k], q.inv[k], q.offC[k]), -1.0f), q.hiC[k]);
       const float f = floorf(t);
-      const float w = t - f;
-      const bool upper = w >= 0.5f;
+      const bool upper = c >= f;
+      wf[k] = t - f;
+      wc[k] = c - (upper ? f : f - 1.0f);
       jf[k] = (int)f;
       jc[k] = upper ? jf[k] : jf[k] - 1;
-      wf[k] = w;
-      wc[k] = w + (upper ? -0.5f : 0.5f);
     }
   }
   __device__ __forceinline__ int entry(const FaceQuads& T, int a) const {

@@ -2,6 +2,8 @@
 edges, one-cell axes, scan chunks, ragged multigrid levels, values that are not
 finite.
 """
+import ctypes
+import ctypes.util
 import threading
 
 import numpy as np
@@ -251,6 +253,54 @@ def test_substep_samples_at_and_beyond_the_grid(cuda, res, rk):
     n = hfgrid.op_advect_particles(res, o, h, [dev(a) for a in v], pd, dt, 1.0, rk, clamp_mode=0)
     assert n == 1
     assert np.abs(host(pd) - ref).max() < 1e-5 * h.max() + 4 * 2.0 ** -24 * np.abs(ref).max()
+
+def test_substep_sample_is_its_formula_to_the_bit(cuda):
+    """A floor and a weight per coordinate, then lerps of the corners along x, y
+    and z, every operation rounded to FP32 once: one Euler substep against that
+    formula, bit for bit.  (The substeps' positions feed the next step's
+    markers, so a weight off in its last bit is another trajectory.)  One
+    coordinate of each particle is small, so that its displacement's last bits
+    are not rounded away with the position's."""
+    fmaf = ctypes.CDLL(ctypes.util.find_library("m")).fmaf
+    fmaf.restype, fmaf.argtypes = ctypes.c_float, [ctypes.c_float] * 3
+    fma = np.vectorize(lambda a, b, c: np.float32(fmaf(a, b, c)), otypes=[np.float32])
+    f32 = np.float32
+    rng = np.random.default_rng(4)
+    res, o, h, dt = (21, 18, 33), np.array((0.3, 0.0, -0.7), f32), np.array((0.11, 0.25, 0.07), f32), f32(0.05)
+    ext = (np.array(res) * h.astype(np.float64))
+    v = [(0.1 * ext[a] / dt * (1 + rng.random(s))).astype(f32) for a, s in enumerate(oracle.face_shapes(res))]
+    pos = 0.75 * rng.random((1500, 3)) * ext
+    pos[np.arange(1500), np.arange(1500) % 3] *= 0.02
+    pos[:30] += rng.choice((-1, 1), (30, 3)) * 0.2 * ext  # beyond the grid: the box clamp makes some of them equal
+    pos = (o + pos).astype(f32)
+    inv = f32(1) / h
+    off = -(o * inv)
+    ref = np.empty_like(pos)
+    for a in range(3):
+        i, w = [], []
+        for k in range(3):
+            n = res[k] + (k == a)
+            t = fma(pos[:, k], inv[k], off[k] if k == a else off[k] - f32(0.5))
+            t = np.minimum(np.maximum(t, f32(-1)), np.nextafter(f32(n), f32(0)))
+            j = np.floor(t)
+            w.append(t - j)
+            j = j.astype(int)
+            i.append((np.clip(j, 0, n - 1), np.clip(j + 1, 0, n - 1)))
+
+        def lerp(w, p, q):
+            return fma(w, q - p, p)
+        at = {(z, y, x): v[a][i[2][z], i[1][y], i[0][x]] for z in (0, 1) for y in (0, 1) for x in (0, 1)}
+        row = {(z, y): lerp(w[0], at[z, y, 0], at[z, y, 1]) for z in (0, 1) for y in (0, 1)}
+        val = lerp(w[2], lerp(w[1], row[0, 0], row[0, 1]), lerp(w[1], row[1, 0], row[1, 1]))
+        top = o[a] + f32(res[a]) * h[a]
+        ref[:, a] = np.maximum(o[a], np.minimum(fma(dt, val, pos[:, a]), top))
+    pd = dev(pos)
+    n = hfgrid.op_advect_particles(res, o, h, [dev(x) for x in v], pd, float(dt), 1e4, 0, clamp_mode=0)
+    assert n == 1
+    got = host(pd)
+    inside = (ref > o) & (ref < o + np.array(res) * h * f32(0.999))  # the box bound itself rounds as an FMA may
+    assert inside.mean() > 0.9
+    assert np.array_equal(got[inside], ref[inside])
 
 
 # --- operator scratch -----------------------------------------------------------------
