@@ -189,6 +189,7 @@ constexpr int kResidentIters = 512;  // iterations the solvers ask of one launch
 bool cgResidentEligible(const Dim3i& cg, int precond, bool xDouble);
 // bytes of its mailboxes (16-byte aligned; cleared by every launch)
 size_t cgResidentBytes(const Dim3i& cg);
+size_t cgResidentBytesMost();  // of any grid, on any device
 cudaError_t launchCgResident(const Dim3i& cg, float sx, float sy, float sz, const CgCode* code, float* r, float* x,
                              float* p, float* zG, void* mailboxes, CgState* st, int precond, const int* sched,
                              int maxIters, cudaStream_t s);

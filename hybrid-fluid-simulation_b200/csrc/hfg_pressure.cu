@@ -1795,10 +1795,11 @@ cudaError_t launchCgCluster(const Dim3i& cg, float sx, float sy, float sz, const
   ResArgs A{cg, sx, sy, sz, code, r, x, p, zG, nullptr, st, maxIters};
   return launchCluster(k, size, RTH, kResClusterBytes, s, A, sched, cgColumns(cg), kResClusterBytes);
 }
-size_t cgResidentBytes(const Dim3i& cg) {
-  const size_t g = residentGrid(cg);
-  return 2 * g * 2 * g * sizeof(Tagged);
-}
+namespace {
+constexpr size_t mailboxBytes(size_t blocks) { return 2 * blocks * 2 * blocks * sizeof(Tagged); }
+}  // namespace
+size_t cgResidentBytes(const Dim3i& cg) { return mailboxBytes(residentGrid(cg)); }
+size_t cgResidentBytesMost() { return mailboxBytes(kResGrid); }
 
 cudaError_t launchCgResident(const Dim3i& cg, float sx, float sy, float sz, const CgCode* code, float* r, float* x,
                              float* p, float* zG, void* mailboxes, CgState* st, int precond, const int* sched,

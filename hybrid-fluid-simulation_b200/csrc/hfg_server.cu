@@ -71,8 +71,9 @@ double percentile(std::vector<double> v, double q) {
 // velocities x2 + FLIP copy, colour / domain double buffers, markers, solid
 // index, stencil code and CG vectors on the pitched grid, P2G accumulators,
 // face corner tables, extrapolation scratch, boundary SDFs, particles) plus
-// the multigrid levels.
-long long sceneBytes(const int res[3], long long particles, int boundaries, int precond, bool sorting = false) {
+// the multigrid levels or the resident CG's mailboxes.
+long long sceneBytes(const int res[3], long long particles, int boundaries, int precond, bool sorting = false,
+                     bool scalars = true) {
   const long long nx = res[0], ny = res[1], nz = res[2];
   const long long N = nx * ny * nz;
   const long long F = (nx + 1) * ny * nz + nx * (ny + 1) * nz + nx * ny * (nz + 1);
@@ -82,12 +83,14 @@ long long sceneBytes(const int res[3], long long particles, int boundaries, int 
   b += N * 4 * (6 + 2);        // colour x2 x3, domain x2
   b += N * 2;                  // markers, solid index
   b += NC * (2 + 1 + 4 * 4);   // code, CG code, x, r, p x2
-  b += F * 8 + N * 8;          // P2G accumulators (faces, cells)
+  b += F * 8;                  // P2G accumulators of the faces
+  if (scalars) b += N * (16 + 4);  // and of the cells: colour and domain, their weight
   b += ((nx + 2) * (ny + 1) * (nz + 2) + (nx + 1) * (ny + 2) * (nz + 2) + (nx + 1) * (ny + 1) * (nz + 3)) * 16;  // corner tables
   b += F * (2 + 4 + 1);        // extrapolation distance, list, neighbour masks
   b += N * 4 * (long long)boundaries;
   b += particles * (4 * 3 * 4 + 4);  // pos, vel, v0, vector scalars, scalar
   if (precond == HFG_PRECOND_MG) b += NC * 4 * 4 + N * 2;  // level-0 z x2, p x2; coarse levels
+  else b += (long long)cgResidentBytesMost();
   if (sorting) b += particles * (16 + 12) + particles / 16;  // radix keys and values x2, gather buffer, digit counts
   b += 64ll << 20;             // partials, state, allocator granularity
   return b;
@@ -150,7 +153,7 @@ class Server {
     r->d = d;
     r->cells = (long long)d.res[0] * d.res[1] * d.res[2];
     r->footprint = sceneBytes(d.res, particlesBound(d), 1 + d.n_spheres, d.options.precond,
-                              d.options.sort_interval > 0);
+                              d.options.sort_interval > 0, d.options.advect_scalars != 0);
     r->submitted = Clock::now();
     std::lock_guard<std::mutex> lk(mu_);
     r->id = ++nextId_;

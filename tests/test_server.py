@@ -23,6 +23,48 @@ def test_scene_bytes_arithmetic():
     assert hfgrid.scene_bytes((64, 64, 64), 0, 1, hfgrid.PRECOND_MG) > b64
 
 
+def test_scene_bytes_counts_the_cell_accumulators():
+    """A carried colour and domain take 20 bytes a cell of P2G accumulators
+    (four sums and a weight).  All else that grows with the cells, on a pitched
+    grid: velocity and its copy 36, colour and domain 32, markers and solid
+    index 2, CG 19, face accumulators 24, corner tables 48, extrapolation 21,
+    one SDF 4."""
+    big, small = (1024, 512, 512), (512, 512, 512)
+    per_cell = (hfgrid.scene_bytes(big, 0) - hfgrid.scene_bytes(small, 0)) / 512 ** 3
+    assert 206 <= per_cell < 209  # what the faces past the last cell add is below 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precond", [hfgrid.PRECOND_JACOBI, hfgrid.PRECOND_MG])
+def test_scene_bytes_covers_what_a_scene_takes(cuda, precond):
+    """Device memory before and after the first steps of a scene whose grid is
+    large beside the estimate's allowance for the allocator (64 MiB)."""
+    import gc
+    import torch
+    res = (256, 256, 256)
+
+    def scene(n, per_cell):
+        s = hfgrid.Solver(1 / 60, n, (0.0, 0.0, 0.0), tuple(1 / k for k in n))
+        s.add_analytic_solid(hfgrid.SOLID_WALLS)
+        s.set_advection(hfgrid.ADV_MIX_PIC_FLIP, hfgrid.RK3, hfgrid.LINEAR, 1.0, 0.05)
+        s.set_options(precond=precond, tol_mode=hfgrid.TOL_RELATIVE, tol=1e-6, max_iter=20, advect_scalars=1)
+        s.generate_fluid_domain_from_bbox((0.0, 0.0, 0.0), (0.3, 0.4, 1.0))
+        s.seed_particles(per_cell, 1)
+        s.update(2)
+        return s
+
+    scene((48, 48, 48), 2)  # the kernels' own memory is taken with their first launch
+    gc.collect()
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    s = scene(res, 2)
+    torch.cuda.synchronize()
+    used = free0 - torch.cuda.mem_get_info()[0]
+    counted = hfgrid.scene_bytes(res, s.num_particles, 1, precond)
+    assert counted - (128 << 20) < used <= counted
+
+
 def test_particles_bound_and_validation():
     import ctypes as C
     d = hfgrid.scene_desc((20, 10, 8), fluid_max=(0.5, 0.5, 1.0), per_cell=8)
