@@ -72,21 +72,29 @@ cudaStream_t st(void* s) { return (cudaStream_t)s; }
 // to the driver at the next synchronisation, and each operator call ends in
 // one, so a call on its own paid for mapping its scratch again: 3.5 of the
 // 5.1 ms of a 160^3 particle advection.  This pool keeps up to kPoolKeep bytes
-// across synchronisations (more is given back as before), gives all of it back
-// when an allocation fails for lack of memory and is retried, and leaves the
-// default pool and its settings alone.  The driver orders reuse between
-// streams and threads, as for the default pool.
+// across synchronisations (more is given back as before) and leaves the
+// default pool and its settings alone.  What it keeps goes back to the driver
+// with hfg_release_scratch, and when an allocation of this library fails for
+// lack of memory (giveBackScratch).  The driver orders reuse between streams
+// and threads, as for the default pool.
 constexpr unsigned long long kPoolKeep = 512ull << 20;
 constexpr int kPoolDevices = 64;
+struct ScratchPools {
+  std::mutex mu;
+  cudaMemPool_t of[kPoolDevices] = {};  // null: not made yet
+};
+ScratchPools& scratchPools() {
+  static ScratchPools* p = new ScratchPools;  // never destroyed: scratch may outlive static destruction
+  return *p;
+}
 cudaError_t scratchPool(cudaMemPool_t* pool) {
-  static std::mutex mu;
-  static cudaMemPool_t pools[kPoolDevices] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= kPoolDevices) return cudaDeviceGetDefaultMemPool(pool, dev);
-  std::lock_guard<std::mutex> lk(mu);
-  if (!pools[dev]) {
+  ScratchPools& all = scratchPools();
+  std::lock_guard<std::mutex> lk(all.mu);
+  if (!all.of[dev]) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -101,12 +109,31 @@ cudaError_t scratchPool(cudaMemPool_t* pool) {
     if (e != cudaSuccess && made) cudaMemPoolDestroy(made);
     cudaThreadExchangeStreamCaptureMode(&mode);
     if (e != cudaSuccess) return e;
-    pools[dev] = made;
+    all.of[dev] = made;
   }
-  *pool = pools[dev];
+  *pool = all.of[dev];
   return cudaSuccess;
 }
+// the current device's pool, null if no operator has run there
+cudaMemPool_t scratchPoolMade() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kPoolDevices) return nullptr;
+  ScratchPools& all = scratchPools();
+  std::lock_guard<std::mutex> lk(all.mu);
+  return all.of[dev];
+}
+}  // namespace
 
+// The stream is waited for first: a pool keeps what was freed until the free
+// has run (nothing to wait for, nor allowed, while it is captured).
+void hfg::giveBackScratch(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone) cudaStreamSynchronize(s);
+  if (cudaMemPool_t pool = scratchPoolMade()) cudaMemPoolTrimTo(pool, 0);
+  cudaGetLastError();
+}
+
+namespace {
 // Stream-ordered scratch for the operator entry points.
 template <class T> struct Scratch {
   T* p = nullptr;
@@ -117,9 +144,8 @@ template <class T> struct Scratch {
     cudaError_t e = scratchPool(&pool);
     if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void**)&p, n * sizeof(T), pool, s);
     if (e == cudaErrorMemoryAllocation) {
-      // what the pools hold unused, back to the driver, then once more
       cudaGetLastError();
-      cudaMemPoolTrimTo(pool, 0);
+      giveBackScratch(s);
       e = cudaMallocFromPoolAsync((void**)&p, n * sizeof(T), pool, s);
     }
     if (e != cudaSuccess) {
@@ -164,6 +190,14 @@ HFG_API int hfg_test_inject_alloc_failure(int after) {
   return guarded([&]() -> int {
     NEED(after >= 0, "invalid arguments");
     g_allocFailAfter.store(after);
+    return HFG_OK;
+  });
+}
+
+HFG_API int hfg_release_scratch(void) {
+  return guarded([&]() -> int {
+    check(cudaDeviceSynchronize(), "sync");
+    if (cudaMemPool_t pool = scratchPoolMade()) check(cudaMemPoolTrimTo(pool, 0), "trim");
     return HFG_OK;
   });
 }

@@ -31,6 +31,11 @@ void check(cudaError_t e, const char* what);
 // as cudaMalloc would (HFG_ERR_NOMEM) without calling it.  Disarmed: 0.
 bool injectedAllocFailure();
 
+// Gives what the operators' scratch pool of the current device keeps unused
+// back to the driver, for an allocation on stream s that failed for lack of
+// memory and will be tried once more.
+void giveBackScratch(cudaStream_t s);
+
 // Owning device array.  With a stream the memory comes from the
 // stream-ordered allocator and is returned with cudaFreeAsync on the same
 // stream, so creating and destroying scenes never synchronises the device
@@ -57,9 +62,16 @@ template <class T> struct DArray {
     release();
     if (count == 0) return;
     if (injectedAllocFailure()) throw CudaError("device allocation failed: injected by the test hook", HFG_ERR_NOMEM);
-    cudaError_t e;
-    if (stream) e = cudaMallocAsync((void**)&p, count * sizeof(T), stream);
-    else e = cudaMalloc((void**)&p, count * sizeof(T));
+    auto take = [&] {
+      return stream ? cudaMallocAsync((void**)&p, count * sizeof(T), stream)
+                    : cudaMalloc((void**)&p, count * sizeof(T));
+    };
+    cudaError_t e = take();
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      giveBackScratch(stream);
+      e = take();
+    }
     if (e != cudaSuccess) {
       p = nullptr;
       throw CudaError(std::string("device allocation failed: ") + cudaGetErrorString(e), HFG_ERR_NOMEM);

@@ -204,6 +204,7 @@ def _signatures(lib):
                                             C.POINTER(C.c_longlong), VP]),
         "hfg_selftest_bounded_waits": (C.c_int, [C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
         "hfg_test_inject_alloc_failure": (C.c_int, [C.c_int]),
+        "hfg_release_scratch": (C.c_int, []),
         "hfg_tune_save": (C.c_int, [C.c_char_p]),
         "hfg_batch_create": (C.c_int, [C.c_int, C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_void_p)]),
         "hfg_batch_step": (C.c_int, [VP, C.c_int, C.c_void_p]),
@@ -243,6 +244,12 @@ def selftest_bounded_waits(wait_ms: int = 20):
     a, b = C.c_int(), C.c_int()
     _check(lib().hfg_selftest_bounded_waits(wait_ms, C.byref(a), C.byref(b)))
     return a.value, b.value
+
+
+def release_scratch():
+    """Give the operators' scratch kept on the current device (512 MiB at most)
+    back to the driver."""
+    _check(lib().hfg_release_scratch())
 
 
 def tune_save(path: str):

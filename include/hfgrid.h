@@ -148,6 +148,13 @@ HFG_API int hfg_selftest_bounded_waits(int wait_ms, int* mbarrier_timed_out, int
  * device allocation of the library from now on fails as cudaMalloc would
  * (HFG_ERR_NOMEM), without calling it.  0 disarms. */
 HFG_API int hfg_test_inject_alloc_failure(int after);
+/* The hfg_op_* calls take their scratch from a memory pool of the library's
+ * own and keep up to 512 MiB of it per device between calls.  This gives what
+ * the current device's pool keeps back to the driver, for other allocators in
+ * the process, after waiting for the device; the next operator call takes its
+ * scratch anew.  (The library's own allocations do the same before they fail
+ * for lack of memory.) */
+HFG_API int hfg_release_scratch(void);
 /* The launch shapes measured by the autotuner (option autotune), as a text
  * file of "cg<0 direction | 1 update> px ny nz zchunk" lines; loading adds to
  * the table and sets *entries.  No reference counterpart. */

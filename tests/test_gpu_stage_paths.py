@@ -339,3 +339,47 @@ def test_operators_on_several_threads_and_streams(cuda):
     torch.cuda.empty_cache()
     torch.cuda.synchronize()
     assert free0 - torch.cuda.mem_get_info()[0] < (512 + 256) << 20
+
+
+def _keep_scratch(cuda):
+    """An operator call whose scratch (0.45 GB of tables) the pool keeps."""
+    res = (200, 200, 176)
+    v = [torch.zeros(s, device=cuda) for s in oracle.face_shapes(res)]
+    p = torch.rand((1000, 3), device=cuda)
+    hfgrid.op_advect_particles(res, (0, 0, 0), tuple(1 / n for n in res), v, p, 1 / 60)
+    del v, p
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+
+
+def test_release_scratch_gives_the_pool_back(cuda):
+    hfgrid.release_scratch()
+    _keep_scratch(cuda)
+    free0 = torch.cuda.mem_get_info()[0]
+    hfgrid.release_scratch()
+    assert torch.cuda.mem_get_info()[0] - free0 > 300 << 20
+    _keep_scratch(cuda)  # the next call takes it anew
+
+
+def test_kept_scratch_does_not_refuse_a_scene(cuda):
+    """A scene that fits the free memory and what the pool keeps, but not the
+    free memory alone: its allocations get the pool's."""
+    res = (200, 200, 176)
+    h = tuple(1 / n for n in res)
+    hfgrid.release_scratch()
+    hfgrid.Solver(1 / 60, res, (0, 0, 0), h)  # what the constructor leaves behind the first time
+    _keep_scratch(cuda)
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    hfgrid.release_scratch()
+    kept = torch.cuda.mem_get_info()[0] - free0
+    s = hfgrid.Solver(1 / 60, res, (0, 0, 0), h)
+    need = free0 + kept - torch.cuda.mem_get_info()[0]
+    del s
+    assert kept > 300 << 20 and need > kept
+    _keep_scratch(cuda)
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - need + kept // 2, dtype=torch.uint8, device=cuda)
+    s = hfgrid.Solver(1 / 60, res, (0, 0, 0), h)
+    s.synchronize()
+    del s, hold
+    torch.cuda.empty_cache()
