@@ -6,6 +6,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -26,6 +27,8 @@ int fail(int code, const std::string& msg) {
 }
 
 std::atomic<int> g_allocFailAfter{0};
+std::mutex g_testLeaseMu;
+std::unique_ptr<CoopLease> g_testLease;
 
 template <class F> int guarded(F&& f) {
   try {
@@ -190,6 +193,20 @@ HFG_API int hfg_test_inject_alloc_failure(int after) {
   return guarded([&]() -> int {
     NEED(after >= 0, "invalid arguments");
     g_allocFailAfter.store(after);
+    return HFG_OK;
+  });
+}
+
+HFG_API int hfg_test_hold_lease(int kind) {
+  return guarded([&]() -> int {
+    NEED(kind >= 0 && kind <= 2, "invalid arguments");
+    std::lock_guard<std::mutex> lk(g_testLeaseMu);
+    g_testLease.reset();
+    if (kind > 0) g_testLease = std::make_unique<CoopLease>(kind == 2);
+    if (g_testLease && !g_testLease->held()) {
+      g_testLease.reset();
+      return fail(HFG_ERR_STATE, "the lease is not free");
+    }
     return HFG_OK;
   });
 }
@@ -789,8 +806,11 @@ int extrapolateGrids(int ngrids, const Dim3i* rc, float* const* vals, int layers
     User() { extrapUsers(+1); }
     ~User() { extrapUsers(-1); }
   } user;
-  CoopLease lease(false);
-  check(launchExtrapLayers(r3, v3, off, sc, layers, s, nullptr), "extrapolation layers");
+  int cluster = 0;
+  check(extrapForm(r3, &cluster), "extrapolation form");
+  std::optional<CoopLease> lease;
+  if (cluster == 0) lease.emplace(false);
+  check(launchExtrapLayers(r3, v3, off, sc, layers, cluster, s, nullptr), "extrapolation layers");
   unsigned int words[4] = {0, 0, 0, 0};
   check(cudaMemcpyAsync(words, extrapBarWords(sc), sizeof(words), cudaMemcpyDeviceToHost, s), "read");
   check(cudaStreamSynchronize(s), "sync");

@@ -808,8 +808,20 @@ CoopLease::~CoopLease() {
 // Whole calls in us, cluster / cooperative grid: 64^3 294 / 400, 96^3 (2.7 M
 // faces) 553 / 581, 128^3 (6.3 M) 927 / 806, 256^3 5333 / 2612; hence the line.
 constexpr long long kExtrapClusterFaces = 3000000;
+cudaError_t extrapForm(const Dim3i rc[3], int* clusterBlocks) {
+  *clusterBlocks = 0;
+  const long long faces = rc[0].size() + rc[1].size() + rc[2].size();
+  if (faces > kExtrapClusterFaces) return cudaSuccess;
+  int size = 0;
+  const cudaError_t e = clusterSize((const void*)kExtrapLayers<true>, kExtrapThreads, 0, &size);
+  if (e != cudaSuccess) return e;
+  // small grids need fewer blocks than the cluster could have
+  while (size > 1 && (long long)(size / 2) * kExtrapThreads * 16 >= faces) size /= 2;
+  *clusterBlocks = size;
+  return cudaSuccess;
+}
 cudaError_t launchExtrapLayers(const Dim3i rc[3], float* const vals[3], const long long off[3], ExtrapScratch sc,
-                               int nums, cudaStream_t s, long long* launches) {
+                               int nums, int clusterBlocks, cudaStream_t s, long long* launches) {
   if (nums <= 1) return cudaSuccess;
   const long long faces = rc[0].size() + rc[1].size() + rc[2].size();
   ExtrapGrids g = extrapGrids(rc, vals, off);
@@ -818,16 +830,10 @@ cudaError_t launchExtrapLayers(const Dim3i rc[3], float* const vals[3], const lo
   const unsigned int* offs = sc.offsets;
   unsigned* bar = extrapBarWords(sc);
   cudaError_t e;
-  if (faces <= kExtrapClusterFaces) {
-    int size = 0;
-    if ((e = clusterSize((const void*)kExtrapLayers<true>, kExtrapThreads, 0, &size)) != cudaSuccess) return e;
-    if (size > 0) {
-      // small grids need fewer blocks than the cluster could have
-      while (size > 1 && (long long)(size / 2) * kExtrapThreads * 16 >= faces) size /= 2;
-      e = launchCluster(kExtrapLayers<true>, size, kExtrapThreads, 0, s, g, mask, list, offs, nums, bar);
-      if (e == cudaSuccess && launches) ++*launches;
-      return e;
-    }
+  if (clusterBlocks > 0) {
+    e = launchCluster(kExtrapLayers<true>, clusterBlocks, kExtrapThreads, 0, s, g, mask, list, offs, nums, bar);
+    if (e == cudaSuccess && launches) ++*launches;
+    return e;
   }
   static std::atomic<int> perSM{0};
   if (perSM.load() == 0) {

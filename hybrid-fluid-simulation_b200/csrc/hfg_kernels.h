@@ -207,11 +207,13 @@ bool cgClusterEligible(const Dim3i& cg, int precond, bool xDouble);
 cudaError_t launchCgCluster(const Dim3i& cg, float sx, float sy, float sz, const CgCode* code, float* r, float* x,
                             float* p, float* zG, CgState* st, int precond, const int* sched, int maxIters,
                             cudaStream_t s);
-// Kernels whose blocks wait on one another must be resident together.  Those
-// that take a share of the GPU (launchExtrapLayers) hold a shared lease from
-// before the launch until the stream has been synchronised after it; one that
-// takes every SM holds the exclusive lease, which is only ever tried for.  The
-// leases are the current device's.
+// Kernels whose blocks wait on one another through memory must be resident
+// together.  Those that take a share of the GPU (launchExtrapLayers as a grid)
+// hold a shared lease from before the launch until the stream has been
+// synchronised after it; one that takes every SM holds the exclusive lease,
+// which is only ever tried for.  A kernel that is one thread block cluster needs
+// neither: the hardware schedules it whole, and it waits on nothing outside
+// itself.  The leases are the current device's.
 class CoopLease {
  public:
   explicit CoopLease(bool exclusive);  // shared: waits for an exclusive holder to finish
@@ -276,8 +278,10 @@ constexpr unsigned kExtrapSmallLayer = 4096;
 // between layers.  The barrier waits are bounded.  Afterwards the words
 // at extrapBarWords() hold kExtrapError (nonzero: a barrier timed out and the
 // layers are incomplete) and kExtrapDepth, the deepest layer filled.
+// clusterBlocks: extrapForm's; 0 launches a grid, under a shared CoopLease.
+cudaError_t extrapForm(const Dim3i rc[3], int* clusterBlocks);
 cudaError_t launchExtrapLayers(const Dim3i rc[3], float* const vals[3], const long long off[3], ExtrapScratch sc,
-                               int nums, cudaStream_t s, long long* launches);
+                               int nums, int clusterBlocks, cudaStream_t s, long long* launches);
 inline unsigned int* extrapBarWords(const ExtrapScratch& sc) { return sc.hist + kMaxLayers + 2; }
 // Registers (+1) or drops (-1) a user of launchExtrapLayers (a solver, an
 // operator call); the launch sizes its grid to a share of the GPU per user.

@@ -8,6 +8,7 @@
 #include <cstring>
 #include <functional>
 #include <mutex>
+#include <optional>
 
 #include "hfg_solver.h"
 
@@ -822,8 +823,11 @@ void GridSolver::extrapolate() {
     long long off[3] = {0, F_[0], F_[0] + F_[1]};
     ExtrapScratch sc{dist_.p, list_.p, hist_.p, offsets_.p, cursor_.p, mask_.p};
     launched(launchExtrapDistance(fr_, vals, off, nums, sc, stream_), "extrapolation distance", 6);
-    CoopLease lease(false);
-    check(launchExtrapLayers(fr_, vals, off, sc, nums, stream_, &launches_), "extrapolation layers");
+    int cluster = 0;
+    check(extrapForm(fr_, &cluster), "extrapolation form");
+    std::optional<CoopLease> lease;
+    if (cluster == 0) lease.emplace(false);
+    check(launchExtrapLayers(fr_, vals, off, sc, nums, cluster, stream_, &launches_), "extrapolation layers");
     readBack(extrapHost_, extrapBarWords(sc), sizeof(unsigned int) * 4, stream_);
     check(cudaStreamSynchronize(stream_), "extrapolation sync");
     if (extrapHost_[kExtrapError] != 0u) throw CudaError("extrapolation: a grid barrier timed out", HFG_ERR_TIMEOUT);

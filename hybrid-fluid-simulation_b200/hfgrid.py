@@ -204,6 +204,7 @@ def _signatures(lib):
                                             C.POINTER(C.c_longlong), VP]),
         "hfg_selftest_bounded_waits": (C.c_int, [C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
         "hfg_test_inject_alloc_failure": (C.c_int, [C.c_int]),
+        "hfg_test_hold_lease": (C.c_int, [C.c_int]),
         "hfg_release_scratch": (C.c_int, []),
         "hfg_tune_save": (C.c_int, [C.c_char_p]),
         "hfg_batch_create": (C.c_int, [C.c_int, C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_void_p)]),
@@ -244,6 +245,12 @@ def selftest_bounded_waits(wait_ms: int = 20):
     a, b = C.c_int(), C.c_int()
     _check(lib().hfg_selftest_bounded_waits(wait_ms, C.byref(a), C.byref(b)))
     return a.value, b.value
+
+
+def hold_lease(kind: int):
+    """For tests: hold the shared (1) or exclusive (2) lease of the device as
+    another scene would, or give it back (0)."""
+    _check(lib().hfg_test_hold_lease(kind))
 
 
 def release_scratch():

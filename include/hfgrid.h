@@ -148,6 +148,12 @@ HFG_API int hfg_selftest_bounded_waits(int wait_ms, int* mbarrier_timed_out, int
  * device allocation of the library from now on fails as cudaMalloc would
  * (HFG_ERR_NOMEM), without calling it.  0 disarms. */
 HFG_API int hfg_test_inject_alloc_failure(int after);
+/* Holds a lease of the current device as another scene would, for tests: 1 the
+ * shared one of the large extrapolations (resident pressure solves are then
+ * refused and take the streaming kernels), 2 the exclusive one of a resident
+ * solve (large extrapolations wait; HFG_ERR_STATE if it is not free), 0 gives
+ * back what is held. */
+HFG_API int hfg_test_hold_lease(int kind);
 /* The hfg_op_* calls take their scratch from a memory pool of the library's
  * own and keep up to 512 MiB of it per device between calls.  This gives what
  * the current device's pool keeps back to the driver, for other allocators in
