@@ -202,7 +202,7 @@ HFG_API int hfg_test_hold_lease(int kind) {
     NEED(kind >= 0 && kind <= 2, "invalid arguments");
     std::lock_guard<std::mutex> lk(g_testLeaseMu);
     g_testLease.reset();
-    if (kind > 0) g_testLease = std::make_unique<CoopLease>(kind == 2);
+    if (kind > 0) g_testLease = kind == 1 ? std::make_unique<CoopLease>(0, 1) : std::make_unique<CoopLease>();
     if (g_testLease && !g_testLease->held()) {
       g_testLease.reset();
       return fail(HFG_ERR_STATE, "the lease is not free");
@@ -741,7 +741,7 @@ HFG_API int hfg_op_project(const int res[3], const float spacing[3], float dt, c
       } while (!host.done && host.resident == 1);
     }
     if (!host.done && cgResidentEligible(cg, init.precond, false)) {
-      CoopLease lease(true);
+      CoopLease lease;
       if (lease.held()) do {
           const cudaError_t e = launchCgResident(cg, sx, sy, sz, cgc, r, x, p0, p1, box, cs, init.precond,
                                                  sched, kResidentIters, s);
@@ -806,11 +806,12 @@ int extrapolateGrids(int ngrids, const Dim3i* rc, float* const* vals, int layers
     User() { extrapUsers(+1); }
     ~User() { extrapUsers(-1); }
   } user;
-  int cluster = 0;
-  check(extrapForm(r3, &cluster), "extrapolation form");
+  ExtrapForm form;
+  check(extrapForm(r3, &form), "extrapolation form");
   std::optional<CoopLease> lease;
-  if (cluster == 0) lease.emplace(false);
-  check(launchExtrapLayers(r3, v3, off, sc, layers, cluster, s, nullptr), "extrapolation layers");
+  if (!form.cluster) lease.emplace(form.blocks, form.slots);
+  check(launchExtrapLayers(r3, v3, off, sc, layers, form.cluster, lease ? lease->blocks() : form.blocks, s, nullptr),
+        "extrapolation layers");
   unsigned int words[4] = {0, 0, 0, 0};
   check(cudaMemcpyAsync(words, extrapBarWords(sc), sizeof(words), cudaMemcpyDeviceToHost, s), "read");
   check(cudaStreamSynchronize(s), "sync");

@@ -769,31 +769,48 @@ namespace {
 std::mutex g_coopMu;
 std::condition_variable g_coopFree;
 struct Coop {
-  int shared = 0;
+  int shared = 0;  // holders of the shared lease, and their blocks
+  int blocks = 0;
   bool exclusive = false;
 };
 std::map<int, Coop> g_coop;  // by device
 }  // namespace
 
-CoopLease::CoopLease(bool exclusive) : exclusive_(exclusive), held_(true), dev_(0) {
+CoopLease::CoopLease() : exclusive_(true) {
+  cudaGetDevice(&dev_);
+  std::lock_guard<std::mutex> lk(g_coopMu);
+  Coop& c = g_coop[dev_];
+  held_ = !c.exclusive && c.shared == 0;
+  if (held_) c.exclusive = true;
+}
+// Up to twice the fair share where that many are free: the users are seldom all
+// here at once.  A call on 256^3 (2.6 ms on the whole GPU) beside 31 idle scenes
+// takes 9.2 ms, on the fair share alone 16.4; 32 threads that extrapolate 112^3
+// at once 6.7 ms for all, on fair shares 8.8.
+CoopLease::CoopLease(int want, int slots) : exclusive_(false), held_(true) {
   cudaGetDevice(&dev_);
   std::unique_lock<std::mutex> lk(g_coopMu);
   Coop& c = g_coop[dev_];
-  if (exclusive) {
-    held_ = !c.exclusive && c.shared == 0;
-    if (held_) c.exclusive = true;
-  } else {
-    g_coopFree.wait(lk, [&] { return !c.exclusive; });
-    ++c.shared;
-  }
+  int fair = 0;
+  g_coopFree.wait(lk, [&] {
+    fair = std::min(want, std::max(1, slots / std::max(1, g_extrapUsers.load())));
+    return !c.exclusive && slots - c.blocks >= fair;
+  });
+  blocks_ = std::min({want, 2 * fair, slots - c.blocks});
+  ++c.shared;
+  c.blocks += blocks_;
 }
 CoopLease::~CoopLease() {
   if (!held_) return;
   {
     std::lock_guard<std::mutex> lk(g_coopMu);
     Coop& c = g_coop[dev_];
-    if (exclusive_) c.exclusive = false;
-    else --c.shared;
+    if (exclusive_) {
+      c.exclusive = false;
+    } else {
+      --c.shared;
+      c.blocks -= blocks_;
+    }
   }
   g_coopFree.notify_all();
 }
@@ -802,52 +819,53 @@ CoopLease::~CoopLease() {
 // of 16 blocks (8 where the device has no 16), whose barrier and values stay
 // within one GPC: a layer of 64^3 takes 3.0 us instead of 4.7; the L2 bandwidth
 // of 16 SMs is what limits it on larger grids.  Those take a cooperative grid: about one
-// block per 4096 faces, at most one per SM, and at most an equal share of the
-// GPU's resident slots for this kernel among the registered users, so that
-// the grids of concurrent scenes always fit on the GPU together.
+// block per 4096 faces, at most one per SM, and at most what its lease grants,
+// so that the grids of concurrent scenes always fit on the GPU together.
 // Whole calls in us, cluster / cooperative grid: 64^3 294 / 400, 96^3 (2.7 M
 // faces) 553 / 581, 128^3 (6.3 M) 927 / 806, 256^3 5333 / 2612; hence the line.
 constexpr long long kExtrapClusterFaces = 3000000;
-cudaError_t extrapForm(const Dim3i rc[3], int* clusterBlocks) {
-  *clusterBlocks = 0;
+cudaError_t extrapForm(const Dim3i rc[3], ExtrapForm* form) {
   const long long faces = rc[0].size() + rc[1].size() + rc[2].size();
-  if (faces > kExtrapClusterFaces) return cudaSuccess;
-  int size = 0;
-  const cudaError_t e = clusterSize((const void*)kExtrapLayers<true>, kExtrapThreads, 0, &size);
-  if (e != cudaSuccess) return e;
-  // small grids need fewer blocks than the cluster could have
-  while (size > 1 && (long long)(size / 2) * kExtrapThreads * 16 >= faces) size /= 2;
-  *clusterBlocks = size;
+  if (faces <= kExtrapClusterFaces) {
+    int size = 0;
+    const cudaError_t e = clusterSize((const void*)kExtrapLayers<true>, kExtrapThreads, 0, &size);
+    if (e != cudaSuccess) return e;
+    // small grids need fewer blocks than the cluster could have
+    while (size > 1 && (long long)(size / 2) * kExtrapThreads * 16 >= faces) size /= 2;
+    if (size > 0) {
+      form->cluster = true;
+      form->blocks = size;
+      return cudaSuccess;
+    }
+  }
+  static std::atomic<int> perSM{0};
+  if (perSM.load() == 0) {
+    int v = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kExtrapLayers<false>, kExtrapThreads, 0);
+    if (e != cudaSuccess) return e;
+    perSM.store(std::max(1, v));
+  }
+  form->cluster = false;
+  form->slots = numSMs() * perSM.load();
+  form->blocks =
+      (int)std::max(1LL, std::min({(faces + 4095) / 4096, (long long)numSMs(), (long long)kExtrapMaxBlocks}));
   return cudaSuccess;
 }
 cudaError_t launchExtrapLayers(const Dim3i rc[3], float* const vals[3], const long long off[3], ExtrapScratch sc,
-                               int nums, int clusterBlocks, cudaStream_t s, long long* launches) {
+                               int nums, bool cluster, int blocks, cudaStream_t s, long long* launches) {
   if (nums <= 1) return cudaSuccess;
-  const long long faces = rc[0].size() + rc[1].size() + rc[2].size();
   ExtrapGrids g = extrapGrids(rc, vals, off);
   const uint8_t* mask = sc.mask;
   const unsigned int* list = sc.list;
   const unsigned int* offs = sc.offsets;
   unsigned* bar = extrapBarWords(sc);
   cudaError_t e;
-  if (clusterBlocks > 0) {
-    e = launchCluster(kExtrapLayers<true>, clusterBlocks, kExtrapThreads, 0, s, g, mask, list, offs, nums, bar);
-    if (e == cudaSuccess && launches) ++*launches;
-    return e;
+  if (cluster) {
+    e = launchCluster(kExtrapLayers<true>, blocks, kExtrapThreads, 0, s, g, mask, list, offs, nums, bar);
+  } else {
+    void* args[] = {&g, &mask, &list, &offs, &nums, &bar};
+    e = cudaLaunchCooperativeKernel((const void*)kExtrapLayers<false>, dim3(blocks), dim3(kExtrapThreads), args, 0, s);
   }
-  static std::atomic<int> perSM{0};
-  if (perSM.load() == 0) {
-    int v = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kExtrapLayers<false>, kExtrapThreads, 0);
-    if (e != cudaSuccess) return e;
-    perSM.store(std::max(1, v));
-  }
-  const long long slots = (long long)numSMs() * perSM.load();
-  const long long share = std::max(1LL, slots / std::max(1, g_extrapUsers.load()));
-  const int blocks = (int)std::max(
-      1LL, std::min({(faces + 4095) / 4096, (long long)numSMs(), share, (long long)kExtrapMaxBlocks}));
-  void* args[] = {&g, &mask, &list, &offs, &nums, &bar};
-  e = cudaLaunchCooperativeKernel((const void*)kExtrapLayers<false>, dim3(blocks), dim3(kExtrapThreads), args, 0, s);
   if (e == cudaSuccess && launches) ++*launches;
   return e;
 }

@@ -209,22 +209,27 @@ cudaError_t launchCgCluster(const Dim3i& cg, float sx, float sy, float sz, const
                             cudaStream_t s);
 // Kernels whose blocks wait on one another through memory must be resident
 // together.  Those that take a share of the GPU (launchExtrapLayers as a grid)
-// hold a shared lease from before the launch until the stream has been
-// synchronised after it; one that takes every SM holds the exclusive lease,
-// which is only ever tried for.  A kernel that is one thread block cluster needs
-// neither: the hardware schedules it whole, and it waits on nothing outside
-// itself.  The leases are the current device's.
+// hold a shared lease on that many of the blocks it holds, from before the
+// launch until the stream has been synchronised after it; one that takes every
+// SM holds the exclusive lease, which is only ever tried for.  A kernel that is
+// one thread block cluster needs neither: the hardware schedules it whole, and
+// it waits on nothing outside itself.  The leases are the current device's.
 class CoopLease {
  public:
-  explicit CoopLease(bool exclusive);  // shared: waits for an exclusive holder to finish
+  CoopLease();  // exclusive, if it is free
+  // Shared, on at most `want` of the `slots` blocks the device holds at once.
+  // Waits while the exclusive lease is held or fewer are free than the fair
+  // share, slots over the registered users (extrapUsers).
+  CoopLease(int want, int slots);
   ~CoopLease();
   bool held() const { return held_; }
+  int blocks() const { return blocks_; }
   CoopLease(const CoopLease&) = delete;
   CoopLease& operator=(const CoopLease&) = delete;
 
  private:
-  bool exclusive_, held_;
-  int dev_;
+  bool exclusive_, held_ = false;
+  int blocks_ = 0, dev_ = 0;
 };
 // Divergence residual of the projected velocity over the fluid cells:
 // *sumOut = sum b^2 (FP64), ticketAndMax[1] = bits of max |b|.  `scratch`
@@ -278,13 +283,18 @@ constexpr unsigned kExtrapSmallLayer = 4096;
 // between layers.  The barrier waits are bounded.  Afterwards the words
 // at extrapBarWords() hold kExtrapError (nonzero: a barrier timed out and the
 // layers are incomplete) and kExtrapDepth, the deepest layer filled.
-// clusterBlocks: extrapForm's; 0 launches a grid, under a shared CoopLease.
-cudaError_t extrapForm(const Dim3i rc[3], int* clusterBlocks);
+// A grid (not form.cluster) is launched under a shared CoopLease on its blocks.
+struct ExtrapForm {
+  bool cluster = false;
+  int blocks = 0;  // of the cluster, or the grid at most
+  int slots = 0;   // grid: blocks of the kernel that the device holds at once
+};
+cudaError_t extrapForm(const Dim3i rc[3], ExtrapForm* form);
 cudaError_t launchExtrapLayers(const Dim3i rc[3], float* const vals[3], const long long off[3], ExtrapScratch sc,
-                               int nums, int clusterBlocks, cudaStream_t s, long long* launches);
+                               int nums, bool cluster, int blocks, cudaStream_t s, long long* launches);
 inline unsigned int* extrapBarWords(const ExtrapScratch& sc) { return sc.hist + kMaxLayers + 2; }
 // Registers (+1) or drops (-1) a user of launchExtrapLayers (a solver, an
-// operator call); the launch sizes its grid to a share of the GPU per user.
+// operator call), for the fair share of a CoopLease.
 void extrapUsers(int delta);
 
 // ---- distance fields --------------------------------------------------------

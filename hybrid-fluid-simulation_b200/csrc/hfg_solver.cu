@@ -678,7 +678,7 @@ bool GridSolver::runCgResident(float sx, float sy, float sz, int pc) {
     } while (!cgHost_->done && cgHost_->resident == 1);
     if (cgHost_->done) return true;
   }
-  CoopLease lease(true);
+  CoopLease lease;
   if (!lease.held()) return false;
   cgBox_.alloc(cgResidentBytes(cg_), stream_);
   do {
@@ -823,11 +823,13 @@ void GridSolver::extrapolate() {
     long long off[3] = {0, F_[0], F_[0] + F_[1]};
     ExtrapScratch sc{dist_.p, list_.p, hist_.p, offsets_.p, cursor_.p, mask_.p};
     launched(launchExtrapDistance(fr_, vals, off, nums, sc, stream_), "extrapolation distance", 6);
-    int cluster = 0;
-    check(extrapForm(fr_, &cluster), "extrapolation form");
+    ExtrapForm form;
+    check(extrapForm(fr_, &form), "extrapolation form");
     std::optional<CoopLease> lease;
-    if (cluster == 0) lease.emplace(false);
-    check(launchExtrapLayers(fr_, vals, off, sc, nums, cluster, stream_, &launches_), "extrapolation layers");
+    if (!form.cluster) lease.emplace(form.blocks, form.slots);
+    check(launchExtrapLayers(fr_, vals, off, sc, nums, form.cluster, lease ? lease->blocks() : form.blocks, stream_,
+                             &launches_),
+          "extrapolation layers");
     readBack(extrapHost_, extrapBarWords(sc), sizeof(unsigned int) * 4, stream_);
     check(cudaStreamSynchronize(stream_), "extrapolation sync");
     if (extrapHost_[kExtrapError] != 0u) throw CudaError("extrapolation: a grid barrier timed out", HFG_ERR_TIMEOUT);

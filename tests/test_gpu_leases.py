@@ -169,3 +169,30 @@ def test_long_solve_of_a_cluster(cuda, precond):
     assert s0["cg_iterations"] == s1["cg_iterations"] > 520
     assert s0["cg_residual"] == pytest.approx(s1["cg_residual"], rel=1e-9)
     assert np.abs(p0 - p1).max() <= s0["cg_iterations"] * 2.0 ** -24 * np.abs(p1).max()
+
+
+def test_idle_scenes_leave_their_share_to_an_extrapolation(cuda):
+    """31 scenes that are not extrapolating: a call takes twice the fair 32nd of
+    the GPU.  A layer is bound by the latency of a block's chain, so a sixteenth
+    costs some twice the time of the whole GPU here, and a 32nd four times."""
+    res = (160, 160, 160)
+    shapes = hfgrid.face_shapes(res)
+    v0 = [torch.full(s, float(UNKNOWN), device=cuda) for s in shapes]
+    for a in v0:
+        a[:, :96, :64] = 1.0
+
+    def best():
+        t = []
+        for _ in range(7):
+            v = [a.clone() for a in v0]
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            hfgrid.op_extrapolate_fc(res, v, 1000)
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    alone = best()
+    idle = [hfgrid.Solver(1 / 60, (4, 4, 4)) for _ in range(31)]
+    assert best() < 3 * alone
+    for s in idle:
+        s.close()
