@@ -1104,7 +1104,7 @@ int fluidSideSdf(const int res[3], const float* density, const float* solid_sdf,
     NEED(validRes(res) && density && solid_sdf && out && distance >= 0 && distance <= 100000, "invalid arguments");
     Dim3i r = toRes(res);
     cudaStream_t s = st(stream);
-    Scratch<int> steps(r.size(), s);
+    Scratch<int> steps(sideSdfInts(r), s);
     Scratch<unsigned int> changed(kStepFlags, s);
     unsigned int* flags = (unsigned int*)pinnedGet(sizeof(unsigned int) * kStepFlags);
     cudaError_t e = launchFluidSideSdf(r, density, solid_sdf, outside, distance, out, steps.p, changed.p, flags, s);

@@ -304,8 +304,9 @@ constexpr int kStepFlags = 48;
 cudaError_t launchFluidSdf(const Dim3i& r, const float* domain, float* sdf, int layers, int* steps,
                            unsigned int* changed, cudaStream_t s);
 // The hybrid coupler's inside / outside distance fields of a fluid density
-// (hostFlags: kStepFlags pinned words; the stream is synchronised once per
-// few relaxation rounds) and its mixed outside field.
+// (steps: sideSdfInts entries; hostFlags: kStepFlags pinned words; the stream is
+// synchronised once per batch of passes) and its mixed outside field.
+size_t sideSdfInts(const Dim3i& r);
 cudaError_t launchFluidSideSdf(const Dim3i& r, const float* density, const float* solid, bool outside, int distance,
                                float* out, int* steps, unsigned int* changed, unsigned int* hostFlags,
                                cudaStream_t s);

@@ -5,6 +5,7 @@ finite.
 import ctypes
 import ctypes.util
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -89,6 +90,54 @@ def test_side_distance_fields(cuda, res, kind, distance):
         f = hfgrid.op_build_fluid_outside_sdf if outside else hfgrid.op_build_fluid_inside_sdf
         f(res, dev(density), dev(solid), out, distance)
         assert np.array_equal(host(out), ref)
+
+
+def _porous(res, closed, seed):
+    """A seed plane below cells of which a share is closed: walks that wind."""
+    rng = np.random.default_rng(seed)
+    shape = res[::-1]
+    density = np.ones(shape, np.float32)
+    density[:, 0, :] = 0.2
+    solid = np.where(rng.random(shape) < closed, -1.0, 1.0).astype(np.float32)
+    return density, solid
+
+
+@pytest.mark.parametrize("res,closed", [((31, 9, 7), 0.3), ((32, 40, 8), 0.3), ((33, 41, 17), 0.6), ((70, 90, 60), 0.45),
+                                        ((100, 64, 65), 0.2), ((3, 200, 2), 0.1)])
+@pytest.mark.parametrize("distance", [1, 2, 4, 5, 12, 1000])
+def test_side_distance_fields_among_scattered_solids(cuda, res, closed, distance):
+    density, solid = _porous(res, closed, 1)
+    wall = solid < 0
+    seed = (density == np.float32(0.2)) & ~wall
+    d = _steps(seed, wall)
+    sweeps = 1
+    while sweeps < distance and np.float32(sweeps - 0.3 - 1) == np.float32(sweeps - 1 - 0.3):
+        sweeps += 1
+    ref = np.where((d >= 0) & (d < sweeps), np.maximum((d - 0.3).astype(np.float32), 0), UNKNOWN).astype(np.float32)
+    ref[wall] = 0
+    out = torch.empty(res[::-1], device=cuda)
+    hfgrid.op_build_fluid_inside_sdf(res, dev(density), dev(solid), out, distance)
+    got = host(out)
+    assert np.array_equal(got == UNKNOWN, ref == UNKNOWN)
+    assert np.allclose(got, ref, rtol=1e-6)  # the value's rounding; the steps are whole
+
+
+def test_side_distance_field_time_among_scattered_solids(cuda):
+    """Each round of line passes settles one straight piece of a walk; among
+    scattered solids a walk has dozens, and no call may cost dozens of rounds."""
+    def best(closed, distance):
+        density, solid = (dev(a) for a in _porous((128, 128, 128), closed, 1))
+        out = torch.empty_like(density)
+        t = []
+        for _ in range(5):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            hfgrid.op_build_fluid_inside_sdf((128, 128, 128), density, solid, out, distance)
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    open_, winding = best(0.0, 1000), best(0.3, 30)
+    assert winding < 15 * open_, (open_, winding)
 
 
 @pytest.mark.parametrize("res", [(1, 1, 1), (2, 1, 1), (33, 31, 5), (64, 3, 70), (17, 130, 4)])
