@@ -334,7 +334,11 @@ struct LerpSampler {
       c1[k] = min(jc + 1, q.n[k] - 1);
     }
   }
-  // component a of a face field (0-2) or a cell field (3)
+  // Component a of a face field (0-2) or a cell field (3).  CHECKED: corners that
+  // are not finite, or so far apart that their difference is not, are summed by
+  // their weights instead: infinite between equal infinities (whose difference
+  // is not a number), finite wherever the value is.
+  template <bool CHECKED>
   __device__ __forceinline__ float sample(const LerpGrid& q, int a, const float* __restrict__ f) const {
     const unsigned nx = (unsigned)(q.n[0] + (a == 0)), ny = (unsigned)(q.n[1] + (a == 1));
     const unsigned x0 = a == 0 ? f0[0] : c0[0], x1 = a == 0 ? f1[0] : c1[0], y0 = a == 1 ? f0[1] : c0[1],
@@ -348,9 +352,15 @@ struct LerpSampler {
     const float a00 = fmaf(wx, v1 - v0, v0), a01 = fmaf(wx, v3 - v2, v2);
     const float a10 = fmaf(wx, v5 - v4, v4), a11 = fmaf(wx, v7 - v6, v6);
     const float d0 = fmaf(wy, a01 - a00, a00), d1 = fmaf(wy, a11 - a10, a10);
-    return fmaf(wz, d1 - d0, d0);
+    const float v = fmaf(wz, d1 - d0, d0);
+    if (!CHECKED || fabsf(v) <= FLT_MAX) return v;
+    const float ux = 1.f - wx, uy = 1.f - wy, uz = 1.f - wz;
+    const float lo = uy * (ux * v0 + wx * v1) + wy * (ux * v2 + wx * v3);
+    const float hi = uy * (ux * v4 + wx * v5) + wy * (ux * v6 + wx * v7);
+    return uz * lo + wz * hi;
   }
 };
+__device__ __forceinline__ bool notFinite(float v) { return !(fabsf(v) <= FLT_MAX); }
 // The trilinear sample of the substeps, from the corner tables alone.  Every
 // axis has two coordinates, one on the face grid and one on the cell-centred
 // grid, each one FMA and clamped to its table's bounds; one floor serves both:

@@ -2163,7 +2163,9 @@ __global__ void kG2PFace(Geom g, ConstFaceField f, const float* __restrict__ pos
 }
 // LINEAR: one sampler (weights and base indices of each axis formed once, with
 // a reciprocal) serves the three components, 32-bit indices.  7.6 M particles
-// on 160^3: 173 -> 135 us.
+// on 160^3: 173 -> 139 us, 134 with unchecked samples (the check stands between
+// the components' loads; one for all three, which keeps or makes again what the
+// weighted sums need, took 153 to 193).
 template <typename I>
 __global__ void kG2PFaceLinear(const __grid_constant__ LerpGrid lg, ConstFaceField f, const float* __restrict__ pos, long long P,
                                float* __restrict__ out) {
@@ -2171,7 +2173,7 @@ __global__ void kG2PFaceLinear(const __grid_constant__ LerpGrid lg, ConstFaceFie
     const LerpSampler fs(lg, pos[3 * p], pos[3 * p + 1], pos[3 * p + 2]);
     float v[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) v[a] = fs.sample(lg, a, f.c[a]);
+    for (int a = 0; a < 3; ++a) v[a] = fs.sample<true>(lg, a, f.c[a]);
 #pragma unroll
     for (int a = 0; a < 3; ++a) out[3 * p + a] = v[a];
   }
@@ -2246,13 +2248,15 @@ __device__ inline void axpyPt(float a, const float v[3], float p[3]) {
   for (int k = 0; k < 3; ++k) p[k] = fmaf(a, v[k], p[k]);
 }
 
+// SAMP 0 and -1: trilinear, plain and CHECKED; 1 to 4: the cubic samplers
+constexpr int kChecked = -1;
 template <int SAMP>
 __device__ inline void sampleVel(ConstFaceField vel, const Geom& g, const LerpGrid& lg, float px, float py, float pz,
                                  float v[3]) {
-  if (SAMP == 0) {
+  if (SAMP <= 0) {
     const LerpSampler fs(lg, px, py, pz);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) v[a] = fs.sample(lg, a, vel.c[a]);
+    for (int a = 0; a < 3; ++a) v[a] = fs.sample<SAMP == kChecked>(lg, a, vel.c[a]);
   } else {
 #pragma unroll
     for (int a = 0; a < 3; ++a) v[a] = cubicSample<SAMP>(vel.c[a], faceGeom(g, a), px, py, pz);
@@ -2293,15 +2297,38 @@ __device__ inline void backTrace(ConstFaceField vel, const Geom& g, const LerpGr
 __device__ __forceinline__ float slLerp(const LerpGrid& lg, int a, const float* __restrict__ f, const float q[3]) {
   const LerpSampler fs(lg, q[0], q[1], q[2]);
   // a is the block's: three forms with constant index selection
-  return a == 0 ? fs.sample(lg, 0, f) : (a == 1 ? fs.sample(lg, 1, f) : fs.sample(lg, 2, f));
+  return a == 0 ? fs.sample<false>(lg, 0, f) : (a == 1 ? fs.sample<false>(lg, 1, f) : fs.sample<false>(lg, 2, f));
 }
+// A point whose linear result is not finite, again with checked samples (a sample
+// of the velocity that is not finite makes the result so): component a of a face
+// field, or a cell field (3).  A thread goes over its points again for it, and
+// the blocks are held to the registers that the first pass needs: 128^3, RK3,
+// 260 us; with every sample checked 300, with this called as the point is made
+// 273, without any check 258.
+__device__ __noinline__ float slChecked(LerpGrid lg, ConstFaceField vel, int acc, float dt, float px, float py, float pz,
+                                         int a, const float* f) {
+  const float p[3] = {px, py, pz};
+  float q[3];
+  backTrace<kChecked>(vel, Geom{}, lg, dt, acc, p, q);
+  return LerpSampler(lg, q[0], q[1], q[2]).sample<true>(lg, a, f);
+}
+// SemiLagrangian.cpp:60-97 sample points: entry (x, y, z) of the faces of axis
+// a, or of the cells (3)
+__device__ __forceinline__ void slPoint(const Geom& g, int a, int x, int y, int z, float p[3]) {
+  const float fx = a == 0 ? (float)x : __fadd_rn((float)x, 0.5f), fy = a == 1 ? (float)y : __fadd_rn((float)y, 0.5f),
+              fz = a == 2 ? (float)z : __fadd_rn((float)z, 0.5f);
+  p[0] = __fadd_rn(__fmul_rn(fx, g.hx), g.ox);
+  p[1] = __fadd_rn(__fmul_rn(fy, g.hy), g.oy);
+  p[2] = __fadd_rn(__fmul_rn(fz, g.hz), g.oz);
+}
+constexpr int kSLThreads = 128;
 // the planes of this thread: runs of zPer, gridDim.y of them apart
 __device__ __forceinline__ int slFirst(int zPer) { return blockIdx.y * zPer; }
 __device__ __forceinline__ int slNext(int z, int zPer) {
   return (z + 1) % zPer ? z + 1 : z + 1 + ((int)gridDim.y - 1) * zPer;
 }
 template <int SAMP>
-__global__ void kSLFace(Geom g, const __grid_constant__ LerpGrid lg, int zPer, int acc, float dt, ConstFaceField vel, ConstFaceField in, FaceField out, float ax,
+__global__ void __launch_bounds__(kSLThreads, SAMP == 0 ? 8 : 1) kSLFace(Geom g, const __grid_constant__ LerpGrid lg, int zPer, int acc, float dt, ConstFaceField vel, ConstFaceField in, FaceField out, float ax,
                         float ay, float az, int doAdd, float bx, float by, float bz, int doAdd2) {
   const int a = blockIdx.z;
   const unsigned nx = (unsigned)(g.r.x + (a == 0)), ny = (unsigned)(g.r.y + (a == 1)), plane = nx * ny;
@@ -2309,17 +2336,28 @@ __global__ void kSLFace(Geom g, const __grid_constant__ LerpGrid lg, int zPer, i
   const float add = a == 0 ? ax : (a == 1 ? ay : az), add2 = a == 0 ? bx : (a == 1 ? by : bz);
   const float* __restrict__ src = a == 0 ? in.c[0] : (a == 1 ? in.c[1] : in.c[2]);
   float* __restrict__ dst = a == 0 ? out.c[0] : (a == 1 ? out.c[1] : out.c[2]);
+  bool bad = false;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
     const unsigned y = i / nx, x = i - y * nx;
     for (int z = slFirst(zPer); z < nz; z = slNext(z, zPer)) {
-      // SemiLagrangian.cpp:60-97 sample points
-      const float fx = a == 0 ? (float)x : __fadd_rn((float)x, 0.5f), fy = a == 1 ? (float)y : __fadd_rn((float)y, 0.5f),
-                  fz = a == 2 ? (float)z : __fadd_rn((float)z, 0.5f);
-      const float p[3] = {__fadd_rn(__fmul_rn(fx, g.hx), g.ox), __fadd_rn(__fmul_rn(fy, g.hy), g.oy),
-                          __fadd_rn(__fmul_rn(fz, g.hz), g.oz)};
-      float q[3];
+      float p[3], q[3];
+      slPoint(g, a, x, y, z, p);
       backTrace<SAMP>(vel, g, lg, dt, acc, p, q);
       float v = SAMP == 0 ? slLerp(lg, a, src, q) : sampleAlg<SAMP>(src, faceGeom(g, a), q[0], q[1], q[2]);
+      if (doAdd) v = __fadd_rn(add, v);
+      if (doAdd2) v = __fadd_rn(add2, v);
+      dst[(unsigned)z * plane + i] = v;
+      if (SAMP == 0) bad |= notFinite(v);
+    }
+  }
+  if (!bad) return;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
+    const unsigned y = i / nx, x = i - y * nx;
+    for (int z = slFirst(zPer); z < nz; z = slNext(z, zPer)) {
+      if (!notFinite(dst[(unsigned)z * plane + i])) continue;
+      float p[3];
+      slPoint(g, a, x, y, z, p);
+      float v = slChecked(lg, vel, acc, dt, p[0], p[1], p[2], a, src);
       if (doAdd) v = __fadd_rn(add, v);
       if (doAdd2) v = __fadd_rn(add2, v);
       dst[(unsigned)z * plane + i] = v;
@@ -2343,7 +2381,7 @@ cudaError_t launchSLFace(const Geom& g, int acc, float dt, ConstFaceField vel, C
                          const float add[3], int doAdd, const float add2[3], int doAdd2, cudaStream_t s,
                          int sampling) {
 #define HFG_SL_FACE(S)                                                                                              \
-  kSLFace<S><<<planeGrid(g.r, 128, 3, slPlanes(g.r)), 128, 0, s>>>(g, makeLerpGrid(g), slPlanes(g.r), acc, dt, vel, in, out, add[0], add[1], add[2], doAdd, add2[0], \
+  kSLFace<S><<<planeGrid(g.r, kSLThreads, 3, slPlanes(g.r)), kSLThreads, 0, s>>>(g, makeLerpGrid(g), slPlanes(g.r), acc, dt, vel, in, out, add[0], add[1], add[2], doAdd, add2[0], \
                                                     add2[1], add2[2], doAdd2)
   switch (sampling) {
     case 1: HFG_SL_FACE(1); break;
@@ -2361,26 +2399,43 @@ struct CellFields {
   float* out[4];
 };
 template <int SAMP>
-__global__ void kSLCell(Geom g, const __grid_constant__ LerpGrid lg, int zPer, int acc, float dt, ConstFaceField vel, CellFields cf, int nf) {
+__global__ void __launch_bounds__(kSLThreads, SAMP == 0 ? 8 : 1) kSLCell(Geom g, const __grid_constant__ LerpGrid lg, int zPer, int acc, float dt, ConstFaceField vel, CellFields cf, int nf) {
   const unsigned nx = (unsigned)g.r.x, plane = nx * (unsigned)g.r.y;
+  bool bad = false;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
     const unsigned y = i / nx, x = i - y * nx;
     for (int z = slFirst(zPer); z < g.r.z; z = slNext(z, zPer)) {
-      const float p[3] = {__fadd_rn(__fmul_rn(__fadd_rn((float)x, 0.5f), g.hx), g.ox),
-                          __fadd_rn(__fmul_rn(__fadd_rn((float)y, 0.5f), g.hy), g.oy),
-                          __fadd_rn(__fmul_rn(__fadd_rn((float)z, 0.5f), g.hz), g.oz)};
-      float q[3];
+      float p[3], q[3];
+      slPoint(g, 3, x, y, z, p);
       backTrace<SAMP>(vel, g, lg, dt, acc, p, q);
       const unsigned c = (unsigned)z * plane + i;
       if (SAMP == 0) {
         const LerpSampler fs(lg, q[0], q[1], q[2]);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          if (k < nf) cf.out[k][c] = fs.sample(lg, 3, cf.in[k]);
+          if (k < nf) {
+            const float v = fs.sample<false>(lg, 3, cf.in[k]);
+            cf.out[k][c] = v;
+            bad |= notFinite(v);
+          }
       } else {
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           if (k < nf) cf.out[k][c] = sampleAlg<SAMP>(cf.in[k], g, q[0], q[1], q[2]);
+      }
+    }
+  }
+  if (!bad) return;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
+    const unsigned y = i / nx, x = i - y * nx;
+    for (int z = slFirst(zPer); z < g.r.z; z = slNext(z, zPer)) {
+      const unsigned c = (unsigned)z * plane + i;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (k >= nf || !notFinite(cf.out[k][c])) continue;
+        float p[3];
+        slPoint(g, 3, x, y, z, p);
+        cf.out[k][c] = slChecked(lg, vel, acc, dt, p[0], p[1], p[2], 3, cf.in[k]);
       }
     }
   }
@@ -2391,14 +2446,14 @@ cudaError_t launchSLCell(const Geom& g, int acc, float dt, ConstFaceField vel, c
   for (int k = 0; k < nfields && k < 4; ++k) { cf.in[k] = in[k]; cf.out[k] = out[k]; }
   const int nf = nfields < 4 ? nfields : 4;
   const int zPer = slPlanes(g.r);
-  const dim3 grid = planeGrid(g.r, 128, 1, zPer);
+  const dim3 grid = planeGrid(g.r, kSLThreads, 1, zPer);
   const LerpGrid lg = makeLerpGrid(g);
   switch (sampling) {
-    case 1: kSLCell<1><<<grid, 128, 0, s>>>(g, lg, zPer, acc, dt, vel, cf, nf); break;
-    case 2: kSLCell<2><<<grid, 128, 0, s>>>(g, lg, zPer, acc, dt, vel, cf, nf); break;
-    case 3: kSLCell<3><<<grid, 128, 0, s>>>(g, lg, zPer, acc, dt, vel, cf, nf); break;
-    case 4: kSLCell<4><<<grid, 128, 0, s>>>(g, lg, zPer, acc, dt, vel, cf, nf); break;
-    default: kSLCell<0><<<grid, 128, 0, s>>>(g, lg, zPer, acc, dt, vel, cf, nf);
+    case 1: kSLCell<1><<<grid, kSLThreads, 0, s>>>(g, lg, zPer, acc, dt, vel, cf, nf); break;
+    case 2: kSLCell<2><<<grid, kSLThreads, 0, s>>>(g, lg, zPer, acc, dt, vel, cf, nf); break;
+    case 3: kSLCell<3><<<grid, kSLThreads, 0, s>>>(g, lg, zPer, acc, dt, vel, cf, nf); break;
+    case 4: kSLCell<4><<<grid, kSLThreads, 0, s>>>(g, lg, zPer, acc, dt, vel, cf, nf); break;
+    default: kSLCell<0><<<grid, kSLThreads, 0, s>>>(g, lg, zPer, acc, dt, vel, cf, nf);
   }
   return cudaGetLastError();
 }

@@ -212,6 +212,59 @@ def test_p2g_value_not_finite_reaches_its_whole_stencil(cuda):
         assert int((~torch.isfinite(o)).sum()) == 64
 
 
+@pytest.mark.parametrize("special", [np.inf, -np.inf, 3e38, np.nan])
+def test_linear_samples_next_to_values_not_finite(cuda, special):
+    """LINEAR G2P and semi-Lagrangian advection weigh the eight corners: between
+    equal infinities that is the infinity, between large values of both signs it
+    is finite, next to a NaN or between opposite infinities it is NaN."""
+    rng = np.random.default_rng(6)
+    res, h = (9, 8, 7), (0.1, 0.1, 0.1)
+    v = [rng.standard_normal(s).astype(np.float32) for s in oracle.face_shapes(res)]
+    for a in v:
+        a[:, :, :3] = special
+        a[:, :, 3] = special if np.isinf(special) else -special
+        a[:2, :, 6:] = -special
+    cell = ((rng.random((500, 3)) * 0.8 + 0.1) + rng.integers(1, 5, (500, 3))) + 0.5  # weights off 0 and 1 ...
+    cell[:, 0] = rng.integers(1, 8, 500) + 0.1 + 0.3 * rng.random(500)  # ... on both grids
+    cell[:, 1:] = np.floor(cell[:, 1:]) + 0.1 + 0.3 * rng.random((500, 2))
+    pos = (cell * 0.1).astype(np.float32)
+
+    def weigh(f, u):
+        f = f.astype(np.float64)
+        i = [np.floor(t).astype(int) for t in u]
+        w = [t - b for t, b in zip(u, i)]
+        acc = np.zeros(len(u[0]))
+        for c in range(8):
+            d = [c & 1, c >> 1 & 1, c >> 2]
+            j = [np.clip(i[k] + d[k], 0, f.shape[2 - k] - 1) for k in range(3)]
+            acc += np.prod([w[k] if d[k] else 1 - w[k] for k in range(3)], 0) * f[j[2], j[1], j[0]]
+        return acc
+
+    def same(got, ref):
+        assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(np.isinf(got), np.isinf(ref))
+        ok = ~np.isnan(ref)
+        assert np.array_equal(np.sign(got[ok]), np.sign(ref[ok]))
+        ok = np.isfinite(ref)
+        np.testing.assert_allclose(got[ok], ref[ok], rtol=1e-4, atol=1e-5 * max(1, np.abs(ref[ok]).max()))
+
+    with np.errstate(all="ignore"):
+        u = pos.astype(np.float64) / 0.1
+        refs = [weigh(v[a], [u[:, k] - (0.0 if k == a else 0.5) for k in range(3)]) for a in range(3)]
+        out = torch.empty(pos.shape, device=cuda)
+        hfgrid.op_g2p_fc(res, (0, 0, 0), h, [dev(a) for a in v], dev(pos), hfgrid.LINEAR, out)
+        for a in range(3):
+            same(host(out)[:, a], refs[a])
+        # a uniform flow that moves every sample by (0.3, 0.2, 0.25) cells
+        shift, dt = np.array((0.3, 0.2, 0.25)), 0.5
+        flow = [np.full(s, -0.1 * shift[a] / dt, np.float32) for a, s in enumerate(oracle.face_shapes(res))]
+        f = v[0][:, :, :9].copy()
+        fout = torch.empty(res[::-1], device=cuda)
+        hfgrid.op_sl_advect_cc(res, (0, 0, 0), h, dev(f), [dev(a) for a in flow], dt, 0, fout)
+        z, y, x = np.meshgrid(*[np.arange(n) for n in res[::-1]], indexing="ij")
+        ref = weigh(f, [t.reshape(-1) + shift[k] for k, t in enumerate((x, y, z))])
+        same(host(fout).reshape(-1), ref)
+
+
 @pytest.mark.parametrize("alg", [hfgrid.LINEAR, hfgrid.QUADRATIC, hfgrid.CUBIC])
 def test_carried_scalars_match_the_operators(cuda, alg):
     """One step's colour and domain against the transfers of the operators."""
