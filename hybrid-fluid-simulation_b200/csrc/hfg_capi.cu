@@ -764,6 +764,7 @@ HFG_API int hfg_op_project(const int res[3], const float spacing[3], float dt, c
       }
       readState();
     }
+    if (!std::isfinite(host.rr)) check(launchZeroOffFluid(cg, cgc, x, s), "zero");
     if (host.error == 4) return fail(HFG_ERR_STATE, "pressure CG: a work item of the schedule is invalid");
     if (host.error) return fail(HFG_ERR_TIMEOUT, "pressure CG: a wait did not complete in time");
     FaceField vv{{vx, vy, vz}};

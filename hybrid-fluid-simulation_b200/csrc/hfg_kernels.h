@@ -193,6 +193,10 @@ size_t cgResidentBytesMost();  // of any grid, on any device
 cudaError_t launchCgResident(const Dim3i& cg, float sx, float sy, float sz, const CgCode* code, float* r, float* x,
                              float* p, float* zG, void* mailboxes, CgState* st, int precond, const int* sched,
                              int maxIters, cudaStream_t s);
+// x of the cells off the fluid back to 0, for a solve that has run out of
+// numbers: past an exact residual of 0, say, the scalars are 0 / 0, and these
+// kernels update four cells at a time, 0 times a scalar included.
+cudaError_t launchZeroOffFluid(const Dim3i& cg, const CgCode* code, float* x, cudaStream_t s);
 // whether a launch failed because the device, as this context sees it, does not
 // hold the whole grid at once (the error is cleared: the kernel pair solves)
 inline bool cgResidentRefused(cudaError_t e) {

@@ -1822,6 +1822,17 @@ cudaError_t launchCgResident(const Dim3i& cg, float sx, float sy, float sz, cons
   return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(RTH), args, (size_t)dynBytes, s);
 }
 
+namespace {
+__global__ void kZeroOffFluid(long long n, const CgCode* __restrict__ code, float* __restrict__ x) {
+  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
+    if (!(code[c] & 1)) x[c] = 0.f;
+}
+}  // namespace
+cudaError_t launchZeroOffFluid(const Dim3i& cg, const CgCode* code, float* x, cudaStream_t s) {
+  kZeroOffFluid<<<(unsigned)std::min((cg.size() + 255) / 256, 8LL * numSMs()), 256, 0, s>>>(cg.size(), code, x);
+  return cudaGetLastError();
+}
+
 int cgScheduleTarget(int precond, bool xDouble) {
   int per = kSchedPerSM;
   auto take = [&](const void* k) { per = std::min(per, residentBlocks(k)); };

@@ -658,6 +658,7 @@ void GridSolver::runCg() {
   } else {
     const int pc = opt_.precond == HFG_PRECOND_JACOBI ? 1 : 0;
     if (!runCgResident(sx, sy, sz, pc)) runCgChunks(sx, sy, sz, pc);
+    else if (!std::isfinite(cgHost_->rr)) launched(launchZeroOffFluid(cg_, cgc_.p, cgx_.p, stream_), "zero");
   }
   if (cgHost_->error == 4) throw CudaError("pressure CG: a work item of the schedule is invalid", HFG_ERR_STATE);
   if (cgHost_->error) throw CudaError("pressure CG: a wait did not complete in time", HFG_ERR_TIMEOUT);

@@ -91,3 +91,28 @@ def test_cg_iterate_vs_fp64(cuda, res, fill, precond):
     err = float((p.double() - ref).norm() / ref.norm())
     assert err < 1e-4, err
     assert bool((p[mk != 1] == 0).all())
+
+
+@pytest.mark.parametrize("res", [(5, 3, 2), (40, 20, 12), (128, 96, 100), (200, 160, 150)])
+@pytest.mark.parametrize("precond", [0, 1])
+def test_cells_off_the_fluid_stay_zero_when_a_solve_breaks_down(cuda, res, precond):
+    """Past an exact solution (a tolerance of 0 asks for more iterations) the CG's
+    scalars are 0 / 0: no number comes out at the fluid's cells, but air and
+    solid keep pressure 0.  One fluid cell in each quad of four, each a system
+    of its own that one iteration solves; 600 iterations are two launches."""
+    nx, ny, nz = res
+    mk = torch.zeros((nz, ny, nx), dtype=torch.uint8, device=cuda)
+    mk[::2, ::2, 1::4] = 1
+    v = [torch.zeros(s, device=cuda) for s in hfgrid.face_shapes(res)]
+    v[0][::2, ::2, 1::4] = 1.0  # the same inflow into every fluid cell, from its left face
+    v[0][:, :, 0] = 0.0
+    sv = [torch.zeros_like(t) for t in v]
+    for iters in (1, 3, 600):
+        p = torch.full(mk.shape, 7.0, device=cuda)
+        w = [t.clone() for t in v]
+        st = hfgrid.op_project(res, (1 / 8, 1 / 8, 1 / 8), DT, mk, w, sv, precond=precond, tol_mode=1, tol=0.0,
+                               max_iter=iters, p_out=p)
+        assert st["iterations"] == iters
+        assert bool((p[mk == 0] == 0).all())
+        if iters == 600:
+            assert bool(torch.isnan(p[mk == 1]).any())
