@@ -32,6 +32,12 @@ inline int gridFor(long long n, int threads = kThreads, int perSM = 16) {
 #define HFG_FOR(i, n) \
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (long long)gridDim.x * blockDim.x)
 
+// The same loop with a 32-bit index that does not step past n: n may lie within
+// a step of 2^32.
+#define HFG_FOR_U(i, n)                                                                                       \
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x, i##Step = gridDim.x * blockDim.x, i##On = i < (n); \
+       i##On; i##On = (n)-i > i##Step, i += i##Step)
+
 // The same loop with an index of type I.  The particle kernels take I = int
 // when 3 n and n + the grid's thread count stay below 2^31, which saves the
 // 64-bit index and address arithmetic of every iteration.
@@ -386,8 +392,8 @@ __global__ void kDistRows(const __grid_constant__ ExtrapGrids g, uint16_t* __res
   const float* __restrict__ val = g.v[blockIdx.y];
   uint16_t* __restrict__ d = dist + g.off[blockIdx.y];
   const int lane = threadIdx.x & 31;
-  const int rows = r.y * r.z, nw = (int)(gridDim.x * blockDim.x) >> 5;
-  for (int row = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += nw) {
+  const long long rows = (long long)r.y * r.z, nw = (gridDim.x * blockDim.x) >> 5;
+  for (long long row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += nw) {
     uint16_t* q = d + (size_t)row * r.x;
     const float* p = val + (size_t)row * r.x;
     int carry = BIG;
@@ -433,7 +439,7 @@ __global__ void kDistCols(const __grid_constant__ ExtrapGrids g, int axis, uint1
   const unsigned stride = axis == 1 ? nx : plane;
   const int len = axis == 1 ? r.y : r.z;
   const unsigned lines = axis == 1 ? nx * (unsigned)r.z : plane;
-  for (unsigned l = blockIdx.x * blockDim.x + threadIdx.x; l < lines; l += gridDim.x * blockDim.x) {
+  HFG_FOR_U(l, lines) {
     unsigned base = l;
     if (axis == 1) {
       const unsigned z = l / nx;
@@ -479,11 +485,11 @@ __global__ void kDistCols(const __grid_constant__ ExtrapGrids g, int axis, uint1
 }
 
 // Histogram of layers 1..nums-1 (layers >= nums stay UNKNOWN).
-__global__ void kDistHist(unsigned n, const uint16_t* __restrict__ d, int nums, unsigned int* __restrict__ hist) {
+__global__ void kDistHist(long long n, const uint16_t* __restrict__ d, int nums, unsigned int* __restrict__ hist) {
   __shared__ unsigned int sh[kMaxLayers + 1];
   for (int i = threadIdx.x; i <= kMaxLayers; i += blockDim.x) sh[i] = 0;
   __syncthreads();
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  HFG_FOR(i, n) {
     const unsigned v = d[i];
     if (v >= 1 && (int)v < nums) atomicAdd(&sh[v], 1u);
   }
@@ -557,7 +563,8 @@ __global__ void __launch_bounds__(kScatterThreads)
   const uint16_t* __restrict__ d = dist + base;
   __shared__ unsigned int cnt[kMaxLayers + 1], start[kMaxLayers + 1];
   __shared__ int lo, hi;
-  for (unsigned c0 = blockIdx.x * kScatterChunk; c0 < n; c0 += gridDim.x * kScatterChunk) {
+  for (unsigned long long at = blockIdx.x * kScatterChunk; at < n; at += gridDim.x * kScatterChunk) {
+    const unsigned c0 = (unsigned)at;
     if (threadIdx.x == 0) {
       lo = kMaxLayers + 1;
       hi = 0;
@@ -566,8 +573,8 @@ __global__ void __launch_bounds__(kScatterThreads)
     unsigned mn = kMaxLayers + 1, mx = 0;
 #pragma unroll
     for (int k = 0; k < kScatterPer; ++k) {
-      const unsigned i = c0 + k * kScatterThreads + threadIdx.x;
-      const unsigned dv = i < n ? d[i] : 0u;
+      const unsigned o = k * kScatterThreads + threadIdx.x;
+      const unsigned dv = o < n - c0 ? d[c0 + o] : 0u;
       v[k] = dv >= 1 && (int)dv < nums ? dv : 0u;
       if (v[k]) {
         mn = min(mn, dv);
@@ -640,7 +647,7 @@ cudaError_t launchExtrapDistance(const Dim3i rc[3], float* const vals[3], long l
   cudaError_t e = cudaMemsetAsync(sc.hist, 0, sizeof(unsigned int) * kExtrapHistWords, s);
   if (e != cudaSuccess) return e;
   // every block adds its bins to the global ones: few blocks on small grids
-  kDistHist<<<gridFor(total, kThreads, total > 8000000 ? 16 : 4), kThreads, 0, s>>>((unsigned)total, sc.dist, nums, sc.hist);
+  kDistHist<<<gridFor(total, kThreads, total > 8000000 ? 16 : 4), kThreads, 0, s>>>(total, sc.dist, nums, sc.hist);
   kExclusiveScanSmall<<<1, 1024, 0, s>>>(sc.hist, sc.offsets, sc.cursor, kMaxLayers + 1);
   const int blocks =
       (int)std::min<long long>((most + kScatterChunk - 1) / kScatterChunk, (long long)numSMs() * 8);
@@ -917,9 +924,10 @@ __device__ __forceinline__ void markChanged(bool any, unsigned* flag) {
 // of d - lane between closed cells, plus the carry of the chunk before.
 __global__ void kStepsRows(Dim3i r, int* __restrict__ d, unsigned* changed, int round) {
   if (stepsDone(changed, round)) return;
-  const int lane = threadIdx.x & 31, rows = r.y * r.z, nw = (int)(gridDim.x * blockDim.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  const long long rows = (long long)r.y * r.z, nw = (gridDim.x * blockDim.x) >> 5;
   bool any = false;
-  for (int row = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += nw) {
+  for (long long row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += nw) {
     int* q = d + (size_t)row * r.x;
 #pragma unroll
     for (int back = 0; back < 2; ++back) {
@@ -2337,7 +2345,7 @@ __global__ void __launch_bounds__(kSLThreads, SAMP == 0 ? 8 : 1) kSLFace(Geom g,
   const float* __restrict__ src = a == 0 ? in.c[0] : (a == 1 ? in.c[1] : in.c[2]);
   float* __restrict__ dst = a == 0 ? out.c[0] : (a == 1 ? out.c[1] : out.c[2]);
   bool bad = false;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
+  HFG_FOR_U(i, plane) {
     const unsigned y = i / nx, x = i - y * nx;
     for (int z = slFirst(zPer); z < nz; z = slNext(z, zPer)) {
       float p[3], q[3];
@@ -2351,7 +2359,7 @@ __global__ void __launch_bounds__(kSLThreads, SAMP == 0 ? 8 : 1) kSLFace(Geom g,
     }
   }
   if (!bad) return;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
+  HFG_FOR_U(i, plane) {
     const unsigned y = i / nx, x = i - y * nx;
     for (int z = slFirst(zPer); z < nz; z = slNext(z, zPer)) {
       if (!notFinite(dst[(unsigned)z * plane + i])) continue;
@@ -2402,7 +2410,7 @@ template <int SAMP>
 __global__ void __launch_bounds__(kSLThreads, SAMP == 0 ? 8 : 1) kSLCell(Geom g, const __grid_constant__ LerpGrid lg, int zPer, int acc, float dt, ConstFaceField vel, CellFields cf, int nf) {
   const unsigned nx = (unsigned)g.r.x, plane = nx * (unsigned)g.r.y;
   bool bad = false;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
+  HFG_FOR_U(i, plane) {
     const unsigned y = i / nx, x = i - y * nx;
     for (int z = slFirst(zPer); z < g.r.z; z = slNext(z, zPer)) {
       float p[3], q[3];
@@ -2426,7 +2434,7 @@ __global__ void __launch_bounds__(kSLThreads, SAMP == 0 ? 8 : 1) kSLCell(Geom g,
     }
   }
   if (!bad) return;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += gridDim.x * blockDim.x) {
+  HFG_FOR_U(i, plane) {
     const unsigned y = i / nx, x = i - y * nx;
     for (int z = slFirst(zPer); z < g.r.z; z = slNext(z, zPer)) {
       const unsigned c = (unsigned)z * plane + i;
