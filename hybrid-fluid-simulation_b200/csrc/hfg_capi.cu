@@ -923,7 +923,7 @@ HFG_API int hfg_op_p2g_cc(const int res[3], const float origin[3], const float s
     long long N = g.r.size();
     Scratch<float2> acc(N, s);
     check(cudaMemsetAsync(acc.p, 0, 8 * N, s), "memset");
-    check(launchP2GCell(g, alg, pos, val, 1, 0, n, acc.p, s), "p2g");
+    check(launchP2GCell(g, alg, pos, val, n, acc.p, s), "p2g");
     if (normalize) check(launchNormalize(N, acc.p, f, s), "normalize");
     else check(cudaMemcpy2DAsync(f, 4, acc.p, 8, 4, N, cudaMemcpyDeviceToDevice, s), "copy");
     if (w) check(cudaMemcpy2DAsync(w, 4, (const char*)acc.p + 4, 8, 4, N, cudaMemcpyDeviceToDevice, s), "w");

@@ -244,15 +244,6 @@ struct FaceSampler {
     w[0] = x0 * y0 * z0; w[1] = x1 * y0 * z0; w[2] = x0 * y1 * z0; w[3] = x1 * y1 * z0;
     w[4] = x0 * y0 * z1; w[5] = x1 * y0 * z1; w[6] = x0 * y1 * z1; w[7] = x1 * y1 * z1;
   }
-  __device__ __forceinline__ float sample(const Geom& g, int a, const float* __restrict__ f) const {
-    unsigned idx[8];
-    float w[8];
-    corners(g, a, idx, w);
-    float v = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v = fmaf(w[k], __ldg(f + idx[k]), v);
-    return v;
-  }
   // the same trilinear sample from the corner table of the component: two
   // 16-byte loads instead of eight 4-byte ones, reduced by lerps along x,
   // then y, then z (seven FMAs; rounding differs from the weighted sum in the

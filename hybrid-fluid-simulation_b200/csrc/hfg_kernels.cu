@@ -2044,19 +2044,19 @@ cudaError_t launchP2GFace(const Geom& g, int alg, const float* pos, const float*
 }
 
 template <int ALG>
-__global__ void kP2GCell(Geom g, const float* __restrict__ pos, const float* __restrict__ val, int span, int comp,
-                         long long P, float2* acc) {
-  HFG_FOR(p, P) p2gScatter<ALG>(g, pos[3 * p], pos[3 * p + 1], pos[3 * p + 2], val[span * p + comp], acc);
+__global__ void kP2GCell(Geom g, const float* __restrict__ pos, const float* __restrict__ val, long long P,
+                         float2* acc) {
+  HFG_FOR(p, P) p2gScatter<ALG>(g, pos[3 * p], pos[3 * p + 1], pos[3 * p + 2], val[p], acc);
 }
-cudaError_t launchP2GCell(const Geom& g, int alg, const float* pos, const float* val, int span, int comp, long long P,
-                          float2* acc, cudaStream_t s) {
+cudaError_t launchP2GCell(const Geom& g, int alg, const float* pos, const float* val, long long P, float2* acc,
+                          cudaStream_t s) {
   if (P <= 0) return cudaSuccess;
   int gr = gridFor(P);
   switch (alg) {
-    case LINEAR: kP2GCell<LINEAR><<<gr, kThreads, 0, s>>>(g, pos, val, span, comp, P, acc); break;
-    case QUADRATIC: kP2GCell<QUADRATIC><<<gr, kThreads, 0, s>>>(g, pos, val, span, comp, P, acc); break;
-    case CUBIC: kP2GCell<CUBIC><<<gr, kThreads, 0, s>>>(g, pos, val, span, comp, P, acc); break;
-    case P2GSUM: kP2GCell<P2GSUM><<<gr, kThreads, 0, s>>>(g, pos, val, span, comp, P, acc); break;
+    case LINEAR: kP2GCell<LINEAR><<<gr, kThreads, 0, s>>>(g, pos, val, P, acc); break;
+    case QUADRATIC: kP2GCell<QUADRATIC><<<gr, kThreads, 0, s>>>(g, pos, val, P, acc); break;
+    case CUBIC: kP2GCell<CUBIC><<<gr, kThreads, 0, s>>>(g, pos, val, P, acc); break;
+    case P2GSUM: kP2GCell<P2GSUM><<<gr, kThreads, 0, s>>>(g, pos, val, P, acc); break;
     default: break;
   }
   return cudaGetLastError();

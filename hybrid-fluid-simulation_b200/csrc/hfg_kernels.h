@@ -378,8 +378,8 @@ cudaError_t launchSubstepMulti(const SubstepTask* tasks, const long long* chunkS
 cudaError_t launchGatherSubstepStates(const SubstepTask* tasks, int nScenes, int slot, int* out, cudaStream_t s);
 cudaError_t launchP2GFace(const Geom& g, int alg, const float* pos, const float* vel, long long P, float2* acc[3],
                           cudaStream_t s);
-cudaError_t launchP2GCell(const Geom& g, int alg, const float* pos, const float* val, int span, int comp, long long P,
-                          float2* acc, cudaStream_t s);
+cudaError_t launchP2GCell(const Geom& g, int alg, const float* pos, const float* val, long long P, float2* acc,
+                          cudaStream_t s);
 cudaError_t launchNormalize(long long n, const float2* acc, float* out, cudaStream_t s);
 // P2G accumulators of three face grids of F[a] entries in one array: where each
 // starts (an even entry: 16 bytes) and the entries of all
