@@ -171,15 +171,17 @@ def test_extrapolation_bit_exact(cuda):
         assert np.array_equal(host(vd[a]), ref3[a])
 
 
-def test_extrapolation_large_layers_bit_exact(cuda):
-    """Layers far larger than the one-block path takes (kExtrapSmallLayer =
-    4096 entries): a 96^3 face grid known only in a small blob, so the layer
-    at distance d holds ~d^2 faces (up to ~11,900) and the grid-strided path
-    with the bounded grid barrier between layers runs for most of the ~160
-    layers.  Values and
-    the UNKNOWN entries left must equal the oracle's bit for bit."""
+@pytest.mark.parametrize("n", [96, 112])
+def test_extrapolation_large_layers_bit_exact(cuda, n):
+    """Layers far larger than one block takes alone (1024 entries in a cluster,
+    4096 in a grid): face grids known only in a small blob, so the layer at
+    distance d holds ~d^2 faces (up to ~11,900 on 96^3) and most of the ~160 to
+    ~210 layers are spread over the blocks, the first and the last filled by one.
+    96^3 (2.7 M faces) runs as one cluster with its hardware barrier, 112^3
+    (4.3 M) as a grid that meets through mailboxes.  Values and the UNKNOWN
+    entries left must equal the oracle's bit for bit."""
     rng = np.random.default_rng(17)
-    res = (96, 96, 96)
+    res = (n, n, n)
     U = np.finfo(np.float32).max
     v = face_arrays(res, rng)
     for a in range(3):

@@ -181,9 +181,10 @@ def test_extrapolation_shapes(cuda, res):
 @pytest.mark.parametrize("alg", [hfgrid.LINEAR, hfgrid.QUADRATIC, hfgrid.CUBIC])
 @pytest.mark.parametrize("res", [(1, 1, 1), (2, 3, 1), (8, 5, 6), (13, 4, 7)])
 def test_p2g_rows_of_both_alignments(cuda, alg, res):
-    """Rows that start on and off 16 bytes, and rows shorter than the stencil.
-    The sums differ from the FP32 oracle by their order: 64 addends of a face
-    at 2**-24 each, doubled for the weight, stay below 1e-5."""
+    """Rows that start on and off 16 bytes, and rows shorter than the stencil,
+    face by face against the FP64 oracle.  A coordinate of at most 15 cells is off
+    by a few 2**-24 of that, 4e-6 cells, so is each weight, and the FP32 sums add
+    less than 1e-5 of theirs; values, at most 5, weigh as much more."""
     rng = np.random.default_rng(alg)
     h = (0.1, 0.12, 0.09)
     n = 400
@@ -192,6 +193,13 @@ def test_p2g_rows_of_both_alignments(cuda, alg, res):
     out = [torch.empty(s, device=cuda) for s in oracle.face_shapes(res)]
     wgt = [torch.empty(s, device=cuda) for s in oracle.face_shapes(res)]
     hfgrid.op_p2g_fc(res, (0, 0, 0), h, dev(pos), dev(vel), alg, out, wgt)
+    ref, refw = oracle.p2g_fc(res, (0, 0, 0), h, pos, vel, alg, dbl=1)
+    assert np.abs(vel).max() < 5
+    for v, w, rv, rw in zip(out, wgt, ref, refw):
+        c = min(n, 64 * n / w.numel())  # about as many particles reach a face, at most
+        v, w, rv, rw = (a.astype(np.float64) for a in (host(v), host(w), rv, rw))
+        assert (np.abs(w - rw) <= 4e-6 * c + 1e-5 * rw).all()
+        assert (np.abs(v * w - rv * rw) <= 5 * (4e-6 * c + 2e-5 * rw)).all()
     # weights: the sum over all faces of a component is one per particle
     for w in wgt:
         assert abs(float(w.double().sum()) / n - 1) < 1e-5
