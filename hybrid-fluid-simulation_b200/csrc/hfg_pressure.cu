@@ -921,6 +921,10 @@ __global__ void __launch_bounds__(CTX* CTY, 4)
 // CG stage of a 64^3 step 1.43 -> 1.36 ms.  The operations and their order are the marching kernels';
 // neighbours that are solid or outside hold zero and are not loaded, which the
 // cell's code tells without coordinates.
+// This form / the marching kernels, us a CG iteration with its V-cycle: 24^3 55.3 /
+// 59.1, 64^3 80.6 / 84.7, 80^3 (0.51 M cells) 103.5 / 108.4, 96^3 113.0 / 116.3,
+// 112^3 128.3 / 127.5, 128^3 139.2 / 132.7.  The crossing is near 1.2 M cells; the
+// line keeps to sizes where the gain is clear.
 constexpr long long kCgSmallGrid = 1 << 19;          // cells of a small grid, at most
 constexpr int kSmallThreads = 256, kSmallCells = 4;  // cells of a thread
 struct CgNb {
@@ -1775,8 +1779,10 @@ const void* clusterKernel(int precond) {
 }
 }  // namespace
 bool cgClusterEligible(const Dim3i& cg, int precond, bool xDouble) {
-  // the fluid is seldom more than a quarter of the grid's planes; a system
-  // that turns out too large costs one launch and one host read
+  // The fluid is seldom more than a quarter of the grid's planes.  A system that
+  // turns out too large costs one launch and one host read, 28 us a solve; one
+  // that fits gains 1.8 us an iteration at 15 fluid planes, 1.2 at 50, 0.7 at 120
+  // and 0.2 beyond 160 (of 6.4 to 8.3 us for the grid)
   if (!cgResidentEligible(cg, precond, xDouble) ||
       (long long)cgColumns(cg) * cg.z > 4LL * kResCluster * RG * kResKL)
     return false;
