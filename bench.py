@@ -47,9 +47,9 @@ CG_DRAM_BYTES_PER_CELL = (42.556e6 + 0.884e6 + 50.508e6 + 0.303e6) / 224 ** 3
 # Algorithmic bytes of one CFL substep per particle: position and v0 read and
 # written (FP32 xyz each); the corner-table gathers hit L2.
 SUBSTEP_BYTES_PER_PARTICLE = 48.0
-# dram__bytes_read.sum + dram__bytes_write.sum of one kSubstep launch, ncu
-# --set full on the 160^3 dam break (7.57 M particles), per particle
-SUBSTEP_DRAM_BYTES_PER_PARTICLE = (243.88e6 + 133.72e6) / 7565040
+# dram__bytes_read.sum + dram__bytes_write.sum of one kSubstep launch (ncu) on
+# a 160^3 dam break's 7.57 M particles, per particle
+SUBSTEP_DRAM_BYTES_PER_PARTICLE = (234.14e6 + 127.59e6) / 7565040
 UNIT = "Mcell-steps/s"
 
 
@@ -815,12 +815,17 @@ def run_dam_break(args):
                          "algorithmic_bytes_per_launch": sub_bytes,
                          "bytes_per_particle": SUBSTEP_BYTES_PER_PARTICLE, "ms_per_launch": sub_launch_ms,
                          "launches_per_step": conv["substeps"], "peak_source": peak_source,
-                         "cg_pair": {"kernel": "kCgDirection + kCgUpdate (one CG iteration)", "achieved": achieved,
+                         "cg_pair": {"kernel": "kCgDirection + kCgUpdate (one streaming CG iteration, timed back to "
+                                               "back on the last system, whichever kernels solved the step)",
+                                     "achieved": achieved,
+                                     "step_ms_per_iter": stage_ms["cg"] / max(conv["cg_iterations"], 1),
                                      "frac": achieved / hbm, "algorithmic_bytes_per_iter": algo_bytes,
                                      "ms_per_iter": cg_ms, "traffic": CG_DRAM_BYTES_PER_CELL * N,
                                      "traffic_source": "ncu dram__bytes_read+write at 224^3, per cell, scaled",
                                      "dram_frac": CG_DRAM_BYTES_PER_CELL * N / (cg_ms / 1e3) / 1e9 / hbm,
-                                     "note": "the 25 B/cell figure counts every cell; the kernels stream only "
+                                     "note": "step_ms_per_iter is the CG stage of one more step over its iterations, "
+                                             "by kCgResident where the fluid fits the shared memory; "
+                                             "the 25 B/cell figure counts every cell; the kernels stream only "
                                              "the fluid runs of the tile columns (the work list) and store at "
                                              "fluid cells only, so frac can pass 1 while dram_frac stays low"}},
             "clocks": clk,
