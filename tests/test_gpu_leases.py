@@ -53,7 +53,7 @@ def _project(res, system, precond, iters):
 # twice).  Both forms do the same FP32 operations on every cell; their FP64 dot
 # products are summed in another order, and a scalar of the recurrence, once
 # rounded to FP32, differs only if its rounding is decided by a last bit of
-# FP64: at odds of about 2**-29 a scalar, not in these systems.  The longest take
+# FP64: at odds of the order of 2**-26 a scalar, not in these systems.  The longest take
 # more than one launch of the resident form.
 @pytest.mark.parametrize("res,iters", [((128, 96, 100), 1), ((128, 96, 100), 20), ((128, 96, 100), 200),
                                        ((300, 40, 60), 1300), ((200, 160, 150), 1), ((200, 160, 150), 200),
